@@ -68,6 +68,12 @@ def cuda_units():
     # K gradient classes, one unit per partner-1 shell
     for l1 in range(LMAX + 1):
         units.append(("kgrad_%d" % l1, os.path.join(CSRC, "kgrad.cu"), ["-DLSJK_KG_L1=%d" % l1]))
+    # K gradient over unique quartets, one unit per bra class (L1 >= L2)
+    for l1 in range(LMAX + 1):
+        for l2 in range(l1 + 1):
+            units.append(("kxgrad_%d%d" % (l1, l2), os.path.join(CSRC, "kxgrad.cu"),
+                          ["-DLSJK_L1=%d" % l1, "-DLSJK_L2=%d" % l2,
+                           '-DLSJK_XG_HEADER="generated/xgquartets_%d%d.cuh"' % (l1, l2)]))
     # bra Hermite classes 0..2*LMAX, and 2*LMAX+1 for the gradients
     for lb in range(2 * LMAX + 2):
         units.append(("jinst_%d" % lb, os.path.join(CSRC, "jinst.cu"), ["-DLSJK_LB=%d" % lb]))

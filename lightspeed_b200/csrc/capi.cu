@@ -798,13 +798,14 @@ int lsjk_exchange_grad(lsjk_context* ctx, int nterm, const double* scales, const
         lsjk::PairList* p = const_cast<lsjk::PairList*>(&pl->p);
         check_lmax(p);
         if (!p->symm) throw lsjk::Error(LSJK_EINVAL, "IntBox::exchangeGrad: pairlist must be symmetric");
-        lsjk::build_kinv(c, p);   // the exact list's rows (merged twins are a K-build option only)
         const lsjk::Basis* b = p->b1;
         const size_t nD = (size_t) b->nao * b->nao, nG = (size_t) b->natom * 3;
         // all three promises: the reference's fully symmetric routine, which reads D13 alone
         // (intbox.cpp:553-564); otherwise its general routine over D13 and D24
         const bool canon = D13symm && D24symm && Dsame;
         const bool same = canon || D13 == D24;
+        // the exact list's rows (merged twins are a K-build option only)
+        if (!canon) lsjk::build_kinv(c, p);
         c->scratch_reset();
         double* dD = ctx->dev(2 * nD + nG);
         double* dG = dD + 2 * nD;
@@ -817,7 +818,10 @@ int lsjk_exchange_grad(lsjk_context* ctx, int nterm, const double* scales, const
         double* D24c = same ? D13c : lsjk::take<double>(c, (size_t) b->ncart * b->ncart);
         lsjk::pure_to_cart(c, b, b, dD, D13c);
         if (!same) lsjk::pure_to_cart(c, b, b, dD + nD, D24c);
-        lsjk::exchange_grad(c, ew, p, D13c, D24c, D13symm && D24symm, canon, dG, thresp);
+        if (canon)
+            lsjk::exchange_grad_symm(c, ew, p, D13c, dG, thresp);
+        else
+            lsjk::exchange_grad(c, ew, p, D13c, D24c, D13symm && D24symm, dG, thresp);
         LSJK_CUDA(cudaMemcpyAsync(h, dG, sizeof(double) * nG, cudaMemcpyDeviceToHost, c->stream));
         check_kernels(c);
         for (size_t i = 0; i < nG; ++i) G[i] += h[i];

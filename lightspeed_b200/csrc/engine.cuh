@@ -356,9 +356,12 @@ void exchange_build(Context* ctx, const Ewald& ew, const PairList* pl12, const P
 // K nuclear gradient (FP64): G[atom][xyz] += sum D13 d(12|34)/dR D24 over the
 // K-invert quartets of a symmetric pair list (K-invert rows built), Cartesian
 // densities in, device G (natom x 3) accumulated. pairsym: D13 and D24 are both
-// symmetric (each term computed once for itself and its mirror); canon: the
-// quartet screen of the reference's fully symmetric routine (D13 == D24 symmetric).
+// symmetric (each term computed once for itself and its mirror).
 void exchange_grad(Context* ctx, const Ewald& ew, const PairList* pl, const double* D13cart, const double* D24cart,
-                   bool pairsym, bool canon, double* G, float thresp);
+                   bool pairsym, double* G, float thresp);
+// The same for one symmetric density (D13 == D24), with the quartet screen of the
+// reference's fully symmetric routine; needs no K-invert rows.
+void exchange_grad_symm(Context* ctx, const Ewald& ew, const PairList* pl, const double* Dcart, double* G,
+                        float thresp);
 
 } // namespace lsjk

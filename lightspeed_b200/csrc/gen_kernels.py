@@ -13,6 +13,8 @@ ones below a size limit, see j_emitted / k_emitted):
   137-171) written as Boys + Hermite recursion instead of per-root Rys sums;
   both evaluate the same Hermite Coulomb integrals.
 
+* xg_<L1><L2><L3><L4>: one Rys root of the K gradient over unique quartets (gen_xg).
+
 * kq_<L1><L2><L3><L4>: one Rys root of a primitive quartet (12|34): the 2-D
   integrals from the standard Rys vertical recursion
       I(a+1,0) = C00 I(a,0) + a B10 I(a-1,0)
@@ -115,80 +117,84 @@ def gen_j(LB, LK):
 
 # --------------------------------------------------------------------- K ----
 
+def dim_tables(em, dim):
+    """G(a, b, c, d) of one direction: emits the 2-D Rys integrals I(a, c) and the transfers
+    to centres 2 and 4 on demand and returns the name of the entry (None: the constant 1)."""
+    memoI = {}
+    memoG = {}
+    base = "wz" if dim == "z" else None
+
+    def I(a, c):
+        key = (a, c)
+        if key in memoI:
+            return memoI[key]
+        if a == 0 and c == 0:
+            memoI[key] = base  # None means the constant 1
+            return base
+        terms = []
+        if c == 0:
+            p = I(a - 1, 0)
+            terms.append(("c00" + dim, p))
+            if a - 1 > 0:
+                terms.append(("R(%d) * b10" % (a - 1), I(a - 2, 0)))
+        else:
+            p = I(a, c - 1)
+            terms.append(("d00" + dim, p))
+            if c - 1 > 0:
+                terms.append(("R(%d) * b01" % (c - 1), I(a, c - 2)))
+            if a > 0:
+                terms.append(("R(%d) * b00" % a, I(a - 1, c - 1)))
+        name = "i%s_%d_%d" % (dim, a, c)
+        expr = None
+        for coef, src in terms:
+            t = coef if src is None else "%s * %s" % (coef, src)
+            if expr is None:
+                expr = t
+            else:
+                if src is None:
+                    expr = "(%s) + %s" % (expr, coef)
+                else:
+                    expr = "fma(%s, %s, %s)" % (coef, src, expr)
+        em.emit("const R %s = %s;" % (name, expr))
+        memoI[key] = name
+        return name
+
+    def G(a, b, c, d):
+        key = (a, b, c, d)
+        if key in memoG:
+            return memoG[key]
+        if d > 0:
+            hi = G(a, b, c + 1, d - 1)
+            lo = G(a, b, c, d - 1)
+            dd = "cd" + dim
+        elif b > 0:
+            hi = G(a + 1, b - 1, c, d)
+            lo = G(a, b - 1, c, d)
+            dd = "ab" + dim
+        else:
+            name = I(a, c)
+            memoG[key] = name
+            return name
+        name = "g%s_%d_%d_%d_%d" % (dim, a, b, c, d)
+        if lo is None:
+            em.emit("const R %s = %s + %s;" % (name, hi, dd))
+        elif hi is None:
+            em.emit("const R %s = fma(%s, %s, R(1));" % (name, dd, lo))
+        else:
+            em.emit("const R %s = fma(%s, %s, %s);" % (name, dd, lo, hi))
+        memoG[key] = name
+        return name
+
+    return G
+
+
 def gen_k(L1, L2, L3, L4):
     em = Emitter()
     LA, LC = L1 + L2, L3 + L4
     c1, c2, c3, c4 = cart_list(L1), cart_list(L2), cart_list(L3), cart_list(L4)
     N1, N2, N3, N4 = len(c1), len(c2), len(c3), len(c4)
 
-    def dimfuncs(dim):
-        memoI = {}
-        memoG = {}
-        base = "wz" if dim == "z" else None
-
-        def I(a, c):
-            key = (a, c)
-            if key in memoI:
-                return memoI[key]
-            if a == 0 and c == 0:
-                memoI[key] = base  # None means the constant 1
-                return base
-            terms = []
-            if c == 0:
-                p = I(a - 1, 0)
-                terms.append(("c00" + dim, p))
-                if a - 1 > 0:
-                    terms.append(("R(%d) * b10" % (a - 1), I(a - 2, 0)))
-            else:
-                p = I(a, c - 1)
-                terms.append(("d00" + dim, p))
-                if c - 1 > 0:
-                    terms.append(("R(%d) * b01" % (c - 1), I(a, c - 2)))
-                if a > 0:
-                    terms.append(("R(%d) * b00" % a, I(a - 1, c - 1)))
-            name = "i%s_%d_%d" % (dim, a, c)
-            expr = None
-            for coef, src in terms:
-                t = coef if src is None else "%s * %s" % (coef, src)
-                if expr is None:
-                    expr = t
-                else:
-                    if src is None:
-                        expr = "(%s) + %s" % (expr, coef)
-                    else:
-                        expr = "fma(%s, %s, %s)" % (coef, src, expr)
-            em.emit("const R %s = %s;" % (name, expr))
-            memoI[key] = name
-            return name
-
-        def G(a, b, c, d):
-            key = (a, b, c, d)
-            if key in memoG:
-                return memoG[key]
-            if d > 0:
-                hi = G(a, b, c + 1, d - 1)
-                lo = G(a, b, c, d - 1)
-                dd = "cd" + dim
-            elif b > 0:
-                hi = G(a + 1, b - 1, c, d)
-                lo = G(a, b - 1, c, d)
-                dd = "ab" + dim
-            else:
-                name = I(a, c)
-                memoG[key] = name
-                return name
-            name = "g%s_%d_%d_%d_%d" % (dim, a, b, c, d)
-            if lo is None:
-                em.emit("const R %s = %s + %s;" % (name, hi, dd))
-            elif hi is None:
-                em.emit("const R %s = fma(%s, %s, R(1));" % (name, dd, lo))
-            else:
-                em.emit("const R %s = fma(%s, %s, %s);" % (name, dd, lo, hi))
-            memoG[key] = name
-            return name
-
-        return G
-
+    dimfuncs = lambda dim: dim_tables(em, dim)
     Gx, Gy, Gz = dimfuncs("x"), dimfuncs("y"), dimfuncs("z")
 
     def mul(a, b):
@@ -226,6 +232,72 @@ def gen_k(L1, L2, L3, L4):
           "    (void)cdx; (void)cdy; (void)cdz;\n"
     return head + pre + "\n".join(em.lines) + "\n}\n"
 
+# ------------------------------------------------------------ K gradient ----
+
+def gen_xg(L1, L2, L3, L4):
+    """One Rys root of the bra-centre derivatives of (12|34), contracted with
+        W = Dac D_bd + Dbc D_ad   (a, b = functions of 1, 2; c, d of 3, 4).
+    Each Cartesian component is x y z; instead of a product per derivative, the
+    components are accumulated into the adjoints of the 1-D integrals (xb[x-exponents] +=
+    W y z, likewise y and z), and each adjoint then meets its entry's two derivatives
+        2 alpha G(a+1) - a G(a-1)   and   2 beta G(b+1) - b G(b-1):
+    seven operations per component and root against sixteen."""
+    em = Emitter()
+    c1, c2, c3, c4 = cart_list(L1), cart_list(L2), cart_list(L3), cart_list(L4)
+    N3, N4 = len(c3), len(c4)
+    G = [dim_tables(em, d) for d in "xyz"]
+    tuples = [(a, b, c, d) for a in range(L1 + 1) for b in range(L2 + 1) for c in range(L3 + 1)
+              for d in range(L4 + 1)]
+    val = [{t: G[k](*t) for t in tuples} for k in range(3)]
+    seen = set()
+    em.emit("R w, t, u;")
+
+    def add(k, t, expr1, expr2):
+        name = "%sb_%d%d%d%d" % (("xyz"[k],) + t)
+        f = expr1 if expr2 is None else (expr2 if expr1 is None else None)
+        if name not in seen:
+            seen.add(name)
+            em.emit("R %s = %s;" % (name, f if f else "%s * %s" % (expr1, expr2)))
+        elif f:
+            em.emit("%s += %s;" % (name, f))
+        else:
+            em.emit("%s = fma(%s, %s, %s);" % (name, expr1, expr2, name))
+
+    for i1, a in enumerate(c1):
+        for i3, c in enumerate(c3):
+            for i2, b in enumerate(c2):
+                for i4, d in enumerate(c4):
+                    t = [(a[k], b[k], c[k], d[k]) for k in range(3)]
+                    x, y, z = val[0][t[0]], val[1][t[1]], val[2][t[2]]
+                    em.emit("w = fma(Dac[%d], Dbd[%d], Dbc[%d] * Dad[%d]);"
+                            % (i1 * N3 + i3, i2 * N4 + i4, i2 * N3 + i3, i1 * N4 + i4))
+                    em.emit("t = w * %s; u = %s;" % (z, "w" if x is None else "w * " + x))
+                    add(0, t[0], "t", y)
+                    add(1, t[1], "t", x)
+                    add(2, t[2], "u", y)
+    for k, dim in enumerate("xyz"):
+        for t in tuples:
+            name = "%sb_%d%d%d%d" % ((dim,) + t)
+            if name not in seen:
+                continue
+            for g, i, e in (("gA", 0, "a2"), ("gB", 1, "b2")):
+                up = G[k](*[t[j] + (j == i) for j in range(4)])
+                s = "%s * %s" % (e, up)
+                if t[i]:
+                    dn = G[k](*[t[j] - (j == i) for j in range(4)])
+                    n = "R(%d)" % t[i] if dn is None else ("%s" % dn if t[i] == 1 else "R(%d) * %s" % (t[i], dn))
+                    s = "fma(%s, %s, -(%s))" % (e, up, n)
+                em.emit("%s[%d] = fma(%s, %s, %s[%d]);" % (g, k, name, s, g, k))
+    head = ("template <typename R>\n__device__ __forceinline__ void xg_%d%d%d%d(%s)\n{\n" % (L1, L2, L3, L4, XG_ARGS))
+    pre = "    (void)abx; (void)aby; (void)abz; (void)cdx; (void)cdy; (void)cdz; (void)b00; (void)b10; (void)b01;\n" \
+          "    (void)d00x; (void)d00y; (void)d00z;\n"
+    return head + pre + "\n".join(em.lines) + "\n}\n"
+
+
+XG_ARGS = ("R c00x, R c00y, R c00z, R d00x, R d00y, R d00z, R b00, R b10, R b01, R abx, R aby, R abz, "
+           "R cdx, R cdy, R cdz, R wz, R a2, R b2, const R* Dac, const R* Dbd, const R* Dbc, const R* Dad, "
+           "R* gA, R* gB")
+
 
 def nherm(L):
     return (L + 1) * (L + 2) * (L + 3) // 6
@@ -245,6 +317,9 @@ def ncart(L):
 GEN_D = 2
 J_TERMS = 1600
 K_COMBOS = 100
+# K gradient over unique quartets (L1 >= L2, L3 >= L4): straight-line code up to this many Cartesian
+# combinations, above it a quartet per warp
+XG_COMBOS = 200
 
 
 def j_emitted(LB, LK):
@@ -303,6 +378,21 @@ def main():
                                   % (L1, L2, L3, L4, args, L1, L2, L3, L4, call))
             with open(os.path.join(out_dir, "kquartets_%d%d.cuh" % (L1, L2)), "w") as fh:
                 fh.write("\n".join(kparts) + "\n")
+    # K gradient: one header per bra pair (L1 >= L2)
+    for L1 in range(lmax + 1):
+        for L2 in range(L1 + 1):
+            parts = list(head) + ["template <int L1, int L2, int L3, int L4> struct XG { static constexpr bool lane = false; };"]
+            for L3 in range(lmax + 1):
+                for L4 in range(L3 + 1):
+                    if ncart(L1) * ncart(L2) * ncart(L3) * ncart(L4) > XG_COMBOS:
+                        continue
+                    parts.append(gen_xg(L1, L2, L3, L4))
+                    parts.append("template <> struct XG<%d, %d, %d, %d> { static constexpr bool lane = true; template <typename R> "
+                                 "__device__ __forceinline__ static void run(%s) { xg_%d%d%d%d<R>(%s); } };"
+                                 % (L1, L2, L3, L4, XG_ARGS, L1, L2, L3, L4,
+                                    ", ".join(x.split()[-1].lstrip("*") for x in XG_ARGS.split(","))))
+            with open(os.path.join(out_dir, "xgquartets_%d%d.cuh" % (L1, L2)), "w") as fh:
+                fh.write("\n".join(parts) + "\n")
     print("wrote", out_dir)
 
 

@@ -100,9 +100,9 @@ struct KGradArgs {
     const int *r12s, *r12l, *r34s, *r34l;
     const float *b12, *b34;
     const double *kab12, *p12, *ip12, *px12, *py12, *pz12, *ax12, *ay12, *az12, *pe12;
-    const int *cart12, *atom12, *pidx12;
+    const int *cart12, *atom12;
     const double *kab34, *p34, *ip34, *px34, *py34, *pz34, *ax34, *ay34, *az34, *pe34;
-    const int *cart34, *atom34, *pidx34;
+    const int *cart34, *atom34;
     BasisView b2, b4;
     const double* D13;
     int ld13;
@@ -111,12 +111,6 @@ struct KGradArgs {
     double* G;
     const KScalars* sc;
     float thr_lo;               // thresp: quartets with bound12 bound34 max|D24 block| >= thresp
-    // canon != 0: the reference's fully symmetric gradient, whose screen reads the
-    // D block of (max(prim1, prim2), max(prim3, prim4)) for every quartet: dblk holds
-    // max|D block| per primitive pair (nprim x nprim), and the tasks carry the global max
-    const double* dblk;
-    int nprim;
-    int canon;
     // pairsym != 0 (D13 and D24 both symmetric): the tasks have prim2 <= prim4 and
     // a task with prim2 < prim4 stands for itself and its mirror (1,2,3,4) <-> (3,4,1,2),
     // whose terms are equal: its D24 block enters doubled

@@ -22,6 +22,7 @@
 #include "engine.cuh"
 #include "lsjk_device.cuh"
 #include "kargs.cuh"
+#include "kxargs.cuh"
 
 namespace lsjk {
 
@@ -109,7 +110,6 @@ struct TaskGenArgs {
     int* ntask_hi;
     float thredp;
     int split;
-    int global_dmax;               // tasks carry the global max|D| (sc) instead of their block's
 };
 
 // Append one task per lane that wants one to the list of its class c: the
@@ -143,9 +143,7 @@ __global__ void k_task_gen(TaskGenArgs A)
     const int L4 = valid ? A.b4.L[i4] : 0;
     // largest |D24| over the pair's block and the batch's densities
     double dmax = 0.0;
-    if (A.global_dmax) {
-        dmax = __longlong_as_double((long long) A.sc->dmax_bits);
-    } else if (valid) {
+    if (valid) {
         const int c2 = A.b2.cart[i2], c4 = A.b4.cart[i4];
         const int n2 = ncart_of(L2), n4 = ncart_of(L4);
         for (int g = g0; g < g1; ++g)
@@ -474,20 +472,178 @@ void exchange_build(Context* ctx, const Ewald& ew, const PairList* pl12, const P
     }
 }
 
-// The K gradient over the K build's quartet set (exchange_grad.cpp:523-760:
+namespace {
+
+// The pairs of the list for the K gradient over unique quartets (XGradArgs): the shell of
+// larger angular momentum first.
+struct XPairs {
+    double *q, *kab, *P[3], *CD[3], *r;
+    int *cc, *cd, *pa, *pb, *pm;
+};
+
+__global__ void k_xpairs(const int* __restrict__ p1, const int* __restrict__ p2, int n, BasisView b, XPairs X)
+{
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= n) return;
+    const bool swap = b.L[p1[k]] < b.L[p2[k]];
+    const int i = swap ? p2[k] : p1[k], j = swap ? p1[k] : p2[k];
+    const double e1 = b.e[i], e2 = b.e[j], q = e1 + e2, r = e2 / q;
+    const double A[3] = {b.x[i], b.y[i], b.z[i]}, B[3] = {b.x[j], b.y[j], b.z[j]};
+    double R2 = 0.0;
+    for (int d = 0; d < 3; ++d) {
+        const double ab = A[d] - B[d];
+        R2 += ab * ab;
+        X.CD[d][k] = ab;
+        X.P[d][k] = (e1 * A[d] + e2 * B[d]) / q;
+    }
+    X.q[k] = q;
+    X.r[k] = r;
+    X.kab[k] = (i == j ? 0.5 : 1.0) * b.c[i] * b.c[j] * exp(-e1 * r * R2) / q;
+    X.cc[k] = b.cart[i];
+    X.cd[k] = b.cart[j];
+    X.pa[k] = i;
+    X.pb[k] = j;
+    X.pm[k] = max(i, j);
+}
+
+// G[k] += sum over the copies
+__global__ void k_xsum(const double* __restrict__ copies, int ncopy, int n, double* __restrict__ G)
+{
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= n) return;
+    double s = 0.0;
+    for (int c = 0; c < ncopy; ++c) s += copies[(long) c * n + k];
+    G[k] += s;
+}
+
+void launch_xgrad(Context* ctx, const XGradArgs& A, int L1, int L2, int L3, int L4)
+{
+    switch (10 * L1 + L2) {
+    case 0: launch_xgrad_12<0, 0>(ctx, A, L3, L4); break;
+    case 10: launch_xgrad_12<1, 0>(ctx, A, L3, L4); break;
+    case 11: launch_xgrad_12<1, 1>(ctx, A, L3, L4); break;
+    case 20: launch_xgrad_12<2, 0>(ctx, A, L3, L4); break;
+    case 21: launch_xgrad_12<2, 1>(ctx, A, L3, L4); break;
+    case 22: launch_xgrad_12<2, 2>(ctx, A, L3, L4); break;
+    case 30: launch_xgrad_12<3, 0>(ctx, A, L3, L4); break;
+    case 31: launch_xgrad_12<3, 1>(ctx, A, L3, L4); break;
+    case 32: launch_xgrad_12<3, 2>(ctx, A, L3, L4); break;
+    case 33: launch_xgrad_12<3, 3>(ctx, A, L3, L4); break;
+    default: throw Error(LSJK_ENOTSUPP, "K gradient: shell above f");
+    }
+}
+
+} // namespace
+
+// The fully symmetric K gradient (one symmetric density, the reference's
+// exchange_grad.cpp:17-470) over unique quartets; see kxgrad.cu.
+void exchange_grad_symm(Context* ctx, const Ewald& ew, const PairList* pl, const double* Dcart, double* G, float thresp)
+{
+    if (ew.alpha.size() > 4) throw Error(LSJK_EINVAL, "exchange_grad: at most 4 Ewald terms");
+    cudaStream_t s = ctx->stream;
+    const Basis* b = pl->b1;
+    const int n = (int) pl->npair;
+    if (!b->nprim || !n || ew.alpha.empty()) return;
+    KScalars* sc = take<KScalars>(ctx, 1);
+    LSJK_CUDA(cudaMemsetAsync(sc, 0, sizeof(KScalars), s));
+    const long nd = (long) b->ncart * b->ncart, np2 = (long) b->nprim * b->nprim;
+    k_absmax<<<std::min<long>(nblk(nd, 256), 1184), 256, 0, s>>>(Dcart, nd, &sc->dmax_bits);
+    k_kscalars<<<1, 1, 0, s>>>(sc, thresp, pl->max_bound, pl->max_bound);
+    double* dblk = take<double>(ctx, np2);
+    k_prim_blockmax<<<nblk(np2, 256), 256, 0, s>>>(Dcart, b->ncart, b->view(), dblk);
+    XPairs X;
+    for (double** x : {&X.q, &X.kab, &X.P[0], &X.P[1], &X.P[2], &X.CD[0], &X.CD[1], &X.CD[2], &X.r})
+        *x = take<double>(ctx, n);
+    for (int** x : {&X.cc, &X.cd, &X.pa, &X.pb, &X.pm}) *x = take<int>(ctx, n);
+    k_xpairs<<<nblk(n, 256), 256, 0, s>>>(pl->p1.p, pl->p2.p, n, b->view(), X);
+    LSJK_CUDA(cudaGetLastError());
+    ctx->stats.kernel_launches += 4;
+
+    // 32 copies of G: the warps' sums of a bra land on few addresses
+    constexpr int kCopies = 32;
+    const int ng = 3 * b->natom;
+    double* copies = take<double>(ctx, (size_t) kCopies * ng);
+    unsigned* queue = take<unsigned>(ctx, kNCombo);
+    LSJK_CUDA(cudaMemsetAsync(copies, 0, sizeof(double) * kCopies * ng, s));
+    LSJK_CUDA(cudaMemsetAsync(queue, 0, sizeof(unsigned) * kNCombo, s));
+
+    XGradArgs A{};
+    A.q = X.q;
+    A.kab = X.kab;
+    A.r = X.r;
+    for (int d = 0; d < 3; ++d) {
+        A.P[d] = X.P[d];
+        A.CD[d] = X.CD[d];
+    }
+    A.cc = X.cc;
+    A.cd = X.cd;
+    A.pa = X.pa;
+    A.pb = X.pb;
+    A.pm = X.pm;
+    A.bound = pl->bound.p;
+    A.b = b->view();
+    A.D = Dcart;
+    A.ld = b->ncart;
+    A.dblk = dblk;
+    A.G = copies;
+    A.ncopy = kCopies;
+    A.ng = ng;
+    A.sc = sc;
+    A.thr = thresp;
+    A.status = ctx->status.p;
+    A.nterm = (int) ew.alpha.size();
+    for (int t = 0; t < A.nterm; ++t) {
+        A.alpha[t] = ew.alpha[t];
+        A.omega[t] = ew.omega[t];
+    }
+    // ranges of the (L1, L2) and (L2, L1) classes of the list
+    int off[kNL][kNL][2] = {}, cnt[kNL][kNL][2] = {};
+    for (size_t c = 0; c + 1 < pl->cls_off.size(); ++c) {
+        const int L1 = std::max(pl->cls_L1[c], pl->cls_L2[c]), L2 = std::min(pl->cls_L1[c], pl->cls_L2[c]);
+        const int side = pl->cls_L1[c] < pl->cls_L2[c] ? 1 : 0;
+        off[L1][L2][side] = (int) pl->cls_off[c];
+        cnt[L1][L2][side] = (int) (pl->cls_off[c + 1] - pl->cls_off[c]);
+    }
+    fork_aux(ctx);
+    int lane = 0;
+    // heaviest classes first, so their tails overlap the lighter ones
+    for (int L1 = kNL - 1; L1 >= 0; --L1)
+        for (int L2 = L1; L2 >= 0; --L2)
+            for (int L3 = kNL - 1; L3 >= 0; --L3)
+                for (int L4 = L3; L4 >= 0; --L4) {
+                    if (!(cnt[L1][L2][0] + cnt[L1][L2][1]) || !(cnt[L3][L4][0] + cnt[L3][L4][1])) continue;
+                    for (int k = 0; k < 2; ++k) {
+                        A.boff[k] = off[L1][L2][k];
+                        A.bn[k] = cnt[L1][L2][k];
+                        A.koff[k] = off[L3][L4][k];
+                        A.kn[k] = cnt[L3][L4][k];
+                    }
+                    const int NR = (L1 + L2 + L3 + L4 + 1) / 2 + 1;   // one quantum up
+                    A.queue = queue + combo_index(L1, L2, L3, L4);
+                    A.rys = ctx->rys64.p + kRysOffset[NR];
+                    A.asym_t = ctx->rys_asym64.p + NR * LSJK_RYS_NMAX;
+                    A.asym_w = ctx->rys_asym64.p + (LSJK_RYS_NMAX + 1) * LSJK_RYS_NMAX + NR * LSJK_RYS_NMAX;
+                    A.nbin = kRysNbin[NR];
+                    A.tmax = kRysTmax[NR];
+                    OnAux on(ctx, lane++);
+                    launch_xgrad(ctx, A, L1, L2, L3, L4);
+                }
+    join_aux(ctx);
+    k_xsum<<<nblk(ng, 128), 128, 0, s>>>(copies, kCopies, ng, G);
+    LSJK_CUDA(cudaGetLastError());
+    ctx->stats.kernel_launches++;
+}
+
+// The general K gradient over the K build's quartet set (exchange_grad.cpp:523-760:
 // bound12 >= thre12, bound34 >= thre34, bound12 bound34 max|D24 block| >=
 // thresp), every (prim2, prim4) pair and every partner pair -- the D13/D24
 // symmetry flags of the reference's general routine only choose which equal
-// terms it skips and doubles, so the sum is the same without them. `canon`:
-// the reference's fully symmetric routine (D13symm, D24symm and Dsame;
-// exchange_grad.cpp:17-470), which computes one representative per set of
-// equal terms and screens all of them with the representative's D block;
-// the same sum over the same quartets here. `pairsym` (D13 and D24 both
-// symmetric, the reference's D13symm and D24symm): the terms of (1,2,3,4) and
-// (3,4,1,2) are equal, screens included, so only tasks with prim2 <= prim4 run
-// and those with prim2 < prim4 count twice.
+// terms it skips and doubles, so the sum is the same without them. `pairsym` (D13
+// and D24 both symmetric, the reference's D13symm and D24symm): the terms of
+// (1,2,3,4) and (3,4,1,2) are equal, screens included, so only tasks with
+// prim2 <= prim4 run and those with prim2 < prim4 count twice.
 void exchange_grad(Context* ctx, const Ewald& ew, const PairList* pl, const double* D13cart, const double* D24cart,
-                   bool pairsym, bool canon, double* G, float thresp)
+                   bool pairsym, double* G, float thresp)
 {
     if (ew.alpha.size() > 4) throw Error(LSJK_EINVAL, "exchange_grad: at most 4 Ewald terms");
     cudaStream_t s = ctx->stream;
@@ -534,15 +690,6 @@ void exchange_grad(Context* ctx, const Ewald& ew, const PairList* pl, const doub
     T.tasks = tasks;
     for (int c = 0; c < kNCombo; ++c) T.cap_off[c] = off[c];
     T.ntask = ntask;
-    T.global_dmax = canon ? 1 : 0;
-    double* dblk = nullptr;
-    if (canon) {
-        const long np2 = (long) b->nprim * b->nprim;
-        dblk = take<double>(ctx, np2);
-        k_prim_blockmax<<<nblk(np2, 256), 256, 0, s>>>(D24cart, b->ncart, b->view(), dblk);
-        LSJK_CUDA(cudaGetLastError());
-        ctx->stats.kernel_launches++;
-    }
     dim3 grid(b->nprim, nblk(b->nprim, 128));
     k_task_gen<<<grid, 128, 0, s>>>(T);
     LSJK_CUDA(cudaGetLastError());
@@ -578,10 +725,6 @@ void exchange_grad(Context* ctx, const Ewald& ew, const PairList* pl, const doub
                     A.pe12 = A.pe34 = d.pe.p;
                     A.cart12 = A.cart34 = d.pcart.p;
                     A.atom12 = A.atom34 = d.patom.p;
-                    A.pidx12 = A.pidx34 = d.pidx.p;
-                    A.dblk = dblk;
-                    A.nprim = b->nprim;
-                    A.canon = canon ? 1 : 0;
                     A.pairsym = pairsym ? 1 : 0;
                     A.b2 = A.b4 = b->view();
                     A.D13 = D13cart;

@@ -4,7 +4,8 @@
 //
 //   G[atom] += sum_{1234} D13 d(12|34)/dR D24
 //
-// over the K-invert quartets of the K build (kbuild.cu): the same task list of
+// for two densities, or without the symmetry promises (one symmetric density:
+// kxgrad.cu), over the K-invert quartets of the K build (kbuild.cu): the same task list of
 // (prim2, prim4) pairs and the same partner rows, here both in bound order.
 // A warp takes a task, its lanes take 32 partners 3 at a time and walk the
 // partners 1 together. Each quartet's derivatives come from the Rys
@@ -250,7 +251,7 @@ __global__ void __launch_bounds__(128) k_exchange_grad(const __grid_constant__ K
             const bool in3 = cs + lane < n34;
             float b34 = 0.0f;
             double kab34 = 0, q = 1, iq = 1, gamma = 0, Qs[3] = {0, 0, 0}, QC[3] = {0, 0, 0}, Cr[3] = {0, 0, 0};
-            int c3 = 0, atomC = 0, K3 = 0;
+            int c3 = 0, atomC = 0;
             if (in3) {
                 b34 = A.b34[k3];
                 kab34 = A.kab34[k3];
@@ -267,7 +268,6 @@ __global__ void __launch_bounds__(128) k_exchange_grad(const __grid_constant__ K
                 }
                 c3 = A.cart34[k3];
                 atomC = A.atom34[k3];
-                K3 = A.pidx34[k3];
             }
             const bool v3 = in3 && b34 >= thre34;
             float bmax34 = v3 ? b34 : 0.0f;
@@ -289,16 +289,7 @@ __global__ void __launch_bounds__(128) k_exchange_grad(const __grid_constant__ K
                         }
                     atomA = aj;
                 }
-                bool pass = v3 && b12 * b34 >= tlo;
-                if (pass && A.canon) {
-                    // the fully symmetric routine screens each quartet with the D block
-                    // of its representative's primitives 2 and 4 (exchange_grad.cpp:137-217):
-                    // (max(prim1, prim2), max(prim3, prim4)) for a symmetric D
-                    const int K1 = A.pidx12[e];
-                    const int r2 = K1 > i2 ? K1 : i2, r4 = K3 > i4 ? K3 : i4;
-                    pass = (double) (b12 * b34) * A.dblk[(long) r2 * A.nprim + r4] >= (double) A.thr_lo;
-                }
-                if (!pass) continue;
+                if (!(v3 && b12 * b34 >= tlo)) continue;
                 const double P[3] = {A.px12[e], A.py12[e], A.pz12[e]};
                 const double Ar[3] = {A.ax12[e], A.ay12[e], A.az12[e]};
                 const int c1 = A.cart12[e];
@@ -563,17 +554,12 @@ __global__ void __launch_bounds__(128) k_exchange_grad_warp(const __grid_constan
                 QC[d] = Q[d] - Cr[d];
                 Qs[d] = dR[d] - Q[d];
             }
-            const int c3 = A.cart34[k3], atomC = A.atom34[k3], K3 = A.pidx34[k3];
+            const int c3 = A.cart34[k3], atomC = A.atom34[k3];
             double gC[3] = {0, 0, 0};
             for (int j = stripe1; j < n12; j += ns1) {
                 const int e = s12 + j;
                 const float b12 = A.b12[e];
                 if (b12 < thre12 || b12 * b34 < tlo) break;
-                if (A.canon) {
-                    const int K1 = A.pidx12[e];
-                    const int r2 = K1 > i2 ? K1 : i2, r4 = K3 > i4 ? K3 : i4;
-                    if ((double) (b12 * b34) * A.dblk[(long) r2 * A.nprim + r4] < (double) A.thr_lo) continue;
-                }
                 const double P[3] = {A.px12[e], A.py12[e], A.pz12[e]};
                 const double Ar[3] = {A.ax12[e], A.ay12[e], A.az12[e]};
                 const int c1 = A.cart12[e];

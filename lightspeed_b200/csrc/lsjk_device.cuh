@@ -216,6 +216,28 @@ __device__ __forceinline__ void rys_eval(R T, const R* __restrict__ tab, int nbi
     }
 }
 
+// Root i alone of the N-point rule (FP64), for lanes that share a quartet's roots out.
+__device__ __forceinline__ void rys_root(double T, const double* __restrict__ tab, int N, int i, int nbin, double tmax,
+                                         const double* __restrict__ asym_t, const double* __restrict__ asym_w,
+                                         double& t2, double& w)
+{
+    double t;
+    if (T < tmax) {
+        const double u = T * (nbin / tmax);
+        int b = static_cast<int>(u);
+        b = b < nbin - 1 ? b : nbin - 1;
+        const double x = 2.0 * (u - b) - 1.0;
+        t = horner8(tab + 8 * (i * nbin + b), x);
+        const double lw = horner8(tab + 8 * ((N + i) * nbin + b), x);
+        w = N == 1 ? lw : exp(lw);
+    } else {
+        const double r = rsqrt(T);
+        t = asym_t[i] * r;
+        w = asym_w[i] * r;
+    }
+    t2 = t * t;
+}
+
 // Boys values F_0..F_L at T >= LSJK_BOYS_TMAX - (one bin) by the FP64
 // asymptotic form F_0 = sqrt(pi/T)/2 and the upward recursion with the exp(-T)
 // term, rounded to FP32 (the FP32 J path from the last table bin on: over that
