@@ -41,36 +41,51 @@ struct DSet {
     int slots;   // record slots (= n)
 };
 
-__global__ void k_ket_screen(const int* __restrict__ p1, const int* __restrict__ p2,
-                             const float* __restrict__ bound, int n, BasisView b3, BasisView b4,
-                             int symm, DSet D, float thre,
-                             unsigned* __restrict__ key, int* __restrict__ val,
+// The ket pairs of every Hermite class, passed by value; the classes stand one
+// after another in the keys and the sorted order (offset off).
+struct KetTables {
+    const int *p1[kNHerm], *p2[kNHerm];
+    const float* bound[kNHerm];
+    int n[kNHerm], off[kNHerm];
+};
+
+// One launch for every class (grid.y). The key sorts by class, then by the screened
+// bound, largest first, dropped pairs last.
+__global__ void k_ket_screen(KetTables T, BasisView b3, BasisView b4, int symm, DSet D, float thre,
+                             unsigned long long* __restrict__ key, int* __restrict__ val,
                              int* __restrict__ nkept, unsigned* __restrict__ maxbits)
 {
+    const int cls = blockIdx.y;
     int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
-    int i = p1[k], j = p2[k];
-    int a1 = b3.cart[i], a2 = b4.cart[j];
-    int c1 = ncart_of(b3.L[i]), c2 = ncart_of(b4.L[j]);
-    int ld = b4.ncart;
-    // max |D| over the pair block (both triangles if symmetric) and, for a
-    // batched launch, over its densities: the batch screens with the union
-    double v = 0.0;
-    for (int g = 0; g < D.n; ++g) {
-        const double* Dc = D.d[g];
-        for (int x = 0; x < c1; ++x)
-            for (int y = 0; y < c2; ++y) v = fmax(v, fabs(Dc[(long) (a1 + x) * ld + a2 + y]));
-        if (symm)
+    bool keep = false;
+    float B2 = 0.0f;
+    if (k < T.n[cls]) {
+        int i = T.p1[cls][k], j = T.p2[cls][k];
+        int a1 = b3.cart[i], a2 = b4.cart[j];
+        int c1 = ncart_of(b3.L[i]), c2 = ncart_of(b4.L[j]);
+        int ld = b4.ncart;
+        // max |D| over the pair block (both triangles if symmetric) and, for a
+        // batched launch, over its densities: the batch screens with the union
+        double v = 0.0;
+        for (int g = 0; g < D.n; ++g) {
+            const double* Dc = D.d[g];
             for (int x = 0; x < c1; ++x)
-                for (int y = 0; y < c2; ++y) v = fmax(v, fabs(Dc[(long) (a2 + y) * ld + a1 + x]));
+                for (int y = 0; y < c2; ++y) v = fmax(v, fabs(Dc[(long) (a1 + x) * ld + a2 + y]));
+            if (symm)
+                for (int x = 0; x < c1; ++x)
+                    for (int y = 0; y < c2; ++y) v = fmax(v, fabs(Dc[(long) (a2 + y) * ld + a1 + x]));
+        }
+        B2 = (float) (v * (double) T.bound[cls][k]);
+        keep = B2 > thre;
+        key[T.off[cls] + k] = ((unsigned long long) cls << 32) | (keep ? ~__float_as_uint(B2) : 0xffffffffu);
+        val[T.off[cls] + k] = k;
     }
-    float B2 = (float) (v * (double) bound[k]);
-    bool keep = B2 > thre;
-    key[k] = keep ? ~__float_as_uint(B2) : 0xffffffffu;
-    val[k] = k;
-    if (keep) {
-        atomicAdd(nkept, 1);
-        atomicMax(maxbits, __float_as_uint(B2));
+    // the class's count and largest bound, one atomic per warp
+    const unsigned m = __ballot_sync(0xffffffffu, keep);
+    const unsigned mx = __reduce_max_sync(0xffffffffu, keep ? __float_as_uint(B2) : 0u);
+    if (m && (threadIdx.x & 31) == 0) {
+        atomicAdd(&nkept[cls], __popc(m));
+        atomicMax(&maxbits[cls], mx);
     }
 }
 
@@ -190,15 +205,15 @@ __device__ void ket_record(int i, int j, BasisView b3, BasisView b4, bool symm, 
 }
 
 template <int LK>
-__global__ void k_ket_herm(const int* __restrict__ perm, const int* __restrict__ nkept,
-                           const int* __restrict__ p1, const int* __restrict__ p2,
-                           const float* __restrict__ bound, const double* __restrict__ geom,
-                           BasisView b3, BasisView b4, int symm, DSet Dc,
-                           double* __restrict__ rec, float* __restrict__ rec32)
+__global__ void k_ket_herm(const unsigned long long* __restrict__ keys_sorted, const int* __restrict__ perm,
+                           const int* __restrict__ nkept, const int* __restrict__ p1, const int* __restrict__ p2,
+                           const double* __restrict__ geom, BasisView b3, BasisView b4, int symm, DSet Dc,
+                           double* __restrict__ rec, float* __restrict__ rec32, float* __restrict__ kbound)
 {
     const int S = 4 + Dc.slots * nherm_of(LK);
     int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= *nkept) return;
+    kbound[k] = __uint_as_float(~(unsigned) keys_sorted[k]);   // the screened bound, back from its sort key
     int src = perm[k];
     int i = p1[src], j = p2[src];
     int L3 = b3.L[i], L4 = b4.L[j];
@@ -215,15 +230,6 @@ __global__ void k_ket_herm(const int* __restrict__ perm, const int* __restrict__
 #pragma unroll
         for (int t = 0; t < S; ++t) r32[t] = (float) r[t];   // S is runtime: plain loop
     }
-}
-
-// kbound of the sorted ket: recomputed from the sort keys
-__global__ void k_ket_bounds(const unsigned* __restrict__ keys_sorted, const int* __restrict__ nkept,
-                             float* __restrict__ kbound)
-{
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= *nkept) return;
-    kbound[k] = __uint_as_float(~keys_sorted[k]);
 }
 
 // ---- 5. bra Hermite -> Cartesian --------------------------------------------
@@ -544,41 +550,66 @@ KetSet prepare_kets(Context* ctx, const PairList* pl12, const PairList* pl34, co
     K.nket = counts;
     K.nbra = counts + kNHerm;
 
-    // 1. ket screening + sort per Hermite class
+    // 1. ket screening + sort: every Hermite class in one launch and one sort (35 key bits);
+    // a launch and a sort per class (35 launches) took longer than the kernels' work
+    KetTables KT{};
+    int total = 0, nmax = 0;
+    for (int LK = 0; LK < kNHerm; ++LK) {
+        const JBraClass& jk = pl34->jb[LK];
+        KT.p1[LK] = jk.p1.p;
+        KT.p2[LK] = jk.p2.p;
+        KT.bound[LK] = jk.bound.p;
+        KT.n[LK] = jk.n;
+        KT.off[LK] = total;
+        total += jk.n;
+        nmax = std::max(nmax, jk.n);
+    }
+    unsigned long long* key = take<unsigned long long>(ctx, total);
+    unsigned long long* keys = take<unsigned long long>(ctx, total);
+    int* val = take<int>(ctx, total);
+    int* perm = take<int>(ctx, total);
+    if (total) {
+        k_ket_screen<<<dim3(nblk(nmax, 256), kNHerm), 256, 0, s>>>(KT, b3->view(), b4->view(), pl34->symm ? 1 : 0, DS,
+                                                                  thre_ket, key, val, K.nket, maxbits);
+        LSJK_CUDA(cudaGetLastError());
+        // in double buffers: the sort then takes no second copy of its own from the scratch
+        cub::DoubleBuffer<unsigned long long> kb(key, keys);
+        cub::DoubleBuffer<int> vb(val, perm);
+        size_t tmp = 0;
+        LSJK_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp, kb, vb, total, 0, 35, s));
+        void* t = ctx->scratch_take(tmp);
+        LSJK_CUDA(cub::DeviceRadixSort::SortPairs(t, tmp, kb, vb, total, 0, 35, s));
+        keys = kb.Current();
+        perm = vb.Current();
+        ctx->stats.kernel_launches += 5;
+    }
     for (int LK = 0; LK < kNHerm; ++LK) {
         const JBraClass& jk = pl34->jb[LK];
         int n = jk.n;
         if (n == 0) continue;
-        unsigned* key = take<unsigned>(ctx, n);
-        unsigned* keys = take<unsigned>(ctx, n);
-        int* val = take<int>(ctx, n);
-        int* perm = take<int>(ctx, n);
-        k_ket_screen<<<nblk(n, 256), 256, 0, s>>>(jk.p1.p, jk.p2.p, jk.bound.p, n, b3->view(), b4->view(),
-                                                 pl34->symm ? 1 : 0, DS, thre_ket, key, val, K.nket + LK,
-                                                 maxbits + LK);
-        size_t tmp = 0;
-        LSJK_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp, key, keys, val, perm, n, 0, 32, s));
-        void* t = ctx->scratch_take(tmp);
-        LSJK_CUDA(cub::DeviceRadixSort::SortPairs(t, tmp, key, keys, val, perm, n, 0, 32, s));
         double*& krec = K.krec[LK];
         float*& krec32 = K.krec32[LK];
         krec = take<double>(ctx, (long) n * (4 + DS.slots * nherm_of(LK)));
         if (mixed) krec32 = take<float>(ctx, (long) n * (4 + DS.slots * nherm_of(LK)));
         K.kbound[LK] = take<float>(ctx, n);
-        k_ket_bounds<<<nblk(n, 256), 256, 0, s>>>(keys, K.nket + LK, K.kbound[LK]);
-        int* nk = K.nket + LK;
+        const int off = KT.off[LK];
+        auto herm = [&](auto lk) {
+            k_ket_herm<decltype(lk)::value><<<nblk(n, 128), 128, 0, s>>>(
+                keys + off, perm + off, K.nket + LK, jk.p1.p, jk.p2.p, jk.geom.p, b3->view(), b4->view(), pl34->symm,
+                DS, krec, krec32, K.kbound[LK]);
+        };
         switch (LK) {
-        case 0: k_ket_herm<0><<<nblk(n, 128), 128, 0, s>>>(perm, nk, jk.p1.p, jk.p2.p, jk.bound.p, jk.geom.p, b3->view(), b4->view(), pl34->symm, DS, krec, krec32); break;
-        case 1: k_ket_herm<1><<<nblk(n, 128), 128, 0, s>>>(perm, nk, jk.p1.p, jk.p2.p, jk.bound.p, jk.geom.p, b3->view(), b4->view(), pl34->symm, DS, krec, krec32); break;
-        case 2: k_ket_herm<2><<<nblk(n, 128), 128, 0, s>>>(perm, nk, jk.p1.p, jk.p2.p, jk.bound.p, jk.geom.p, b3->view(), b4->view(), pl34->symm, DS, krec, krec32); break;
-        case 3: k_ket_herm<3><<<nblk(n, 128), 128, 0, s>>>(perm, nk, jk.p1.p, jk.p2.p, jk.bound.p, jk.geom.p, b3->view(), b4->view(), pl34->symm, DS, krec, krec32); break;
-        case 4: k_ket_herm<4><<<nblk(n, 128), 128, 0, s>>>(perm, nk, jk.p1.p, jk.p2.p, jk.bound.p, jk.geom.p, b3->view(), b4->view(), pl34->symm, DS, krec, krec32); break;
-        case 5: k_ket_herm<5><<<nblk(n, 128), 128, 0, s>>>(perm, nk, jk.p1.p, jk.p2.p, jk.bound.p, jk.geom.p, b3->view(), b4->view(), pl34->symm, DS, krec, krec32); break;
-        case 6: k_ket_herm<6><<<nblk(n, 128), 128, 0, s>>>(perm, nk, jk.p1.p, jk.p2.p, jk.bound.p, jk.geom.p, b3->view(), b4->view(), pl34->symm, DS, krec, krec32); break;
+        case 0: herm(std::integral_constant<int, 0>{}); break;
+        case 1: herm(std::integral_constant<int, 1>{}); break;
+        case 2: herm(std::integral_constant<int, 2>{}); break;
+        case 3: herm(std::integral_constant<int, 3>{}); break;
+        case 4: herm(std::integral_constant<int, 4>{}); break;
+        case 5: herm(std::integral_constant<int, 5>{}); break;
+        case 6: herm(std::integral_constant<int, 6>{}); break;
         default: throw Error(LSJK_ENOTSUPP, "J: ket Hermite class above 6");
         }
         LSJK_CUDA(cudaGetLastError());
-        ctx->stats.kernel_launches += 7;
+        ctx->stats.kernel_launches++;
     }
 
     // 2. bra truncation counts
@@ -653,11 +684,12 @@ void coulomb_build(Context* ctx, const Ewald& ew, const PairList* pl12, const Pa
             if (ctx->tune.j_chunk[LB][LK] > 0) {
                 A.chunk = ctx->tune.j_chunk[LB][LK];
             } else {
-                // default: kJChunk kets per CTA, halved (down to 64) while the grid would not
-                // give every multiprocessor two CTAs -- small molecules need the parallelism
+                // default: kJChunk kets per CTA, halved (down to 8) while the grid would not
+                // give every multiprocessor two CTAs: a thread walks its chunk serially, so a
+                // small molecule's kernel takes as long as one chunk
                 const long tiles = (jb.n + kJThreads - 1) / kJThreads;
                 int chunk = kJChunk;
-                while (chunk > 64 && tiles * ((jk.n + chunk - 1) / chunk) < 2L * ctx->nsm) chunk >>= 1;
+                while (chunk > 8 && tiles * ((jk.n + chunk - 1) / chunk) < 2L * ctx->nsm) chunk >>= 1;
                 A.chunk = chunk;
             }
             A.ng = ng;
@@ -774,7 +806,7 @@ static void coulomb_grad_bra(Context* ctx, const Ewald& ew, const PairList* pl, 
             A.thredp = thresp;
             int chunk = kJChunk;
             const long tiles = (jb.n + kJThreads - 1) / kJThreads;
-            while (chunk > 64 && tiles * ((jk.n + chunk - 1) / chunk) < 2L * ctx->nsm) chunk >>= 1;
+            while (chunk > 8 && tiles * ((jk.n + chunk - 1) / chunk) < 2L * ctx->nsm) chunk >>= 1;
             A.chunk = chunk;
             A.ng = 1;
             A.slots = 1;
