@@ -26,6 +26,7 @@ struct JArgs {
     int mixed;                // 1: quartets with estimate < thredp run in FP32
     float thredp;
     int chunk;                // ket pairs per CTA (grid.y = ceil(nket / chunk))
+    int tuned;                // chunk was set by the autotuner (or a saved table), not the default rule
     int ng;                   // densities of the build (1..kMaxDens); CTA z covers NG of them
     int slots;                // density blocks per ket record (= ng)
     long jbra_stride;         // distance between the densities' bra accumulators

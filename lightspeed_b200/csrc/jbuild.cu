@@ -683,6 +683,7 @@ void coulomb_build(Context* ctx, const Ewald& ew, const PairList* pl12, const Pa
             A.thredp = thredp;
             if (ctx->tune.j_chunk[LB][LK] > 0) {
                 A.chunk = ctx->tune.j_chunk[LB][LK];
+                A.tuned = 1;
             } else {
                 // default: kJChunk kets per CTA, halved (down to 8) while the grid would not
                 // give every multiprocessor two CTAs: a thread walks its chunk serially, so a
@@ -722,6 +723,7 @@ void coulomb_build(Context* ctx, const Ewald& ew, const PairList* pl12, const Pa
                 float best = 1e30f;
                 for (int c : cand) {
                     T.chunk = c;
+                    T.tuned = 1;
                     float ms = 1e30f;
                     for (int rep = 0; rep < 2; ++rep) {
                         LSJK_CUDA(cudaEventRecord(ctx->ev0, s));
@@ -738,6 +740,7 @@ void coulomb_build(Context* ctx, const Ewald& ew, const PairList* pl12, const Pa
                     }
                 }
                 A.chunk = ctx->tune.j_chunk[LB][LK];
+                A.tuned = 1;
             }
             std::optional<OnAux> on;
             if (par) on.emplace(ctx, lane++);

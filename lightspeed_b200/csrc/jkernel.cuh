@@ -5,6 +5,7 @@
 #include "lsjk_device.cuh"
 #include "generated/jquartets.cuh"
 #include "jargs.cuh"
+#include <atomic>
 
 namespace lsjk {
 
@@ -220,21 +221,45 @@ __global__ void __launch_bounds__(kJThreads) k_coulomb(JArgs A)
 
 // The classes without straight-line code (the largest f classes): a bra pair per
 // warp, FP64. For each ket (bound order, all lanes) the lanes build the Hermite
-// integrals R_tuv in a per-warp shared table -- one shell of (t, u, v) at a time,
-// top shell first, in place, as JQLoop does per thread -- and then each lane
-// contracts its bra components t: jp[t] += sum_u R_{t+u} D_u. A thread-per-pair
-// kernel needs the whole table and the accumulators per thread (several KB),
-// which overflow L1 for 128 threads per CTA.
+// integrals R_tuv in per-warp shared tables, one order n of R^(n) at a time from
+// the previous one's table (two tables in turn, so an order is one pass over its
+// entries and one barrier), and then each lane contracts its bra components t:
+// jp[t] += sum_u R_{t+u} D_u. A thread-per-pair kernel needs the whole table and
+// the accumulators per thread (several KB), which overflow L1 for 128 threads per
+// CTA. Bound by shared-memory accesses: an entry of the recursion reads its sources
+// from a table of positions made once per CTA, and the integrals stand in rows of
+// constant (t, u), so the contraction looks one row up per (u_x, u_y) and walks
+// u_z at consecutive addresses. Decoding positions arithmetically for every entry
+// and term, with a barrier per shell, made this kernel several times slower.
 constexpr int kJWarpPairs = kJThreads / 32;   // bra pairs per CTA
+
+// Position of (t, u, v), t + u + v <= L, with v fastest.
+__host__ __device__ constexpr int row_pos(int L, int t, int u, int v)
+{
+    int p = 0;
+    for (int i = 0; i < t; ++i) p += (L - i + 1) * (L - i + 2) / 2;
+    for (int j = 0; j < u; ++j) p += L - t - j + 1;
+    return p + v;
+}
+
+template <int LB, int LK>
+struct JWarpShared {
+    static constexpr int L = LB + LK, H = nherm_of(L);
+    double boys[LSJK_BOYS_NBIN * 8];
+    double R[kJWarpPairs][2][H];
+    double dk[kJWarpPairs][nherm_of(LK)];
+    ushort4 step[H];                            // (x: position, y, z: its sources, w: direction | factor << 2)
+    unsigned short row[(L + 1) * (L + 1)];      // position of (t, u, 0)
+    uint64_t mbar;
+};
 
 template <int LB, int LK>
 __global__ void __launch_bounds__(kJThreads) k_coulomb_warp(JArgs A)
 {
-    constexpr int L = LB + LK, HB = nherm_of(LB), HK = nherm_of(LK), NT = (HB + 31) / 32;
+    constexpr int L = LB + LK, HB = nherm_of(LB), HK = nherm_of(LK), H = nherm_of(L), NT = (HB + 31) / 32;
     const int S = 4 + A.slots * HK;
-    __shared__ __align__(128) double tab[LSJK_BOYS_NBIN * 8];
-    __shared__ __align__(8) uint64_t mbar;
-    __shared__ double Rall[kJWarpPairs][nherm_of(L)];
+    extern __shared__ __align__(128) unsigned char jwarp_smem[];
+    JWarpShared<LB, LK>& sh = *reinterpret_cast<JWarpShared<LB, LK>*>(jwarp_smem);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int nb = *A.nbra, nk = *A.nket;
     const int g = blockIdx.z;   // the density (one per CTA z)
@@ -242,25 +267,46 @@ __global__ void __launch_bounds__(kJThreads) k_coulomb_warp(JArgs A)
     const int j0 = blockIdx.y * A.chunk;
     if (ib >= nb || j0 >= nk) return;
     if (A.bbound[ib] * A.kbound[j0] < A.thresp) return;
-    if (!stage_bulk(tab, A.boys, sizeof(tab), &mbar, A.status)) return;
+    // the recursion's steps in shell order: R_tuv from its neighbours one and two below
+    // in the first non-zero direction
+    for (int k = threadIdx.x; k < H; k += kJThreads) {
+        int N = 0;
+        while (nherm_of(N) <= k) ++N;
+        const int r = N ? k - nherm_of(N - 1) : 0;
+        int ii = 0;
+        while ((ii + 1) * (ii + 2) / 2 <= r) ++ii;
+        const int t[3] = {N - ii, ii - (r - ii * (ii + 1) / 2), r - ii * (ii + 1) / 2};
+        const int d = t[0] > 0 ? 0 : (t[1] > 0 ? 1 : 2);
+        const int n = t[d];
+        auto below = [&](int by) {
+            return n < by ? 0 : row_pos(L, t[0] - (d == 0 ? by : 0), t[1] - (d == 1 ? by : 0), t[2] - (d == 2 ? by : 0));
+        };
+        sh.step[k] = make_ushort4((unsigned short) row_pos(L, t[0], t[1], t[2]), (unsigned short) below(1),
+                                  (unsigned short) below(2), (unsigned short) (d | (n > 1 ? n - 1 : 0) << 2));
+    }
+    for (int k = threadIdx.x; k < (L + 1) * (L + 1); k += kJThreads) {
+        const int t = k / (L + 1), u = k % (L + 1);
+        sh.row[k] = (unsigned short) (t + u <= L ? row_pos(L, t, u, 0) : 0);
+    }
+    if (!stage_bulk(sh.boys, A.boys, sizeof(sh.boys), &sh.mbar, A.status)) return;   // (with CTA barriers)
     const int i = ib + warp;
-    if (i >= nb) return;   // (after the CTA-wide staging)
-    double* Rb = Rall[warp];
+    if (i >= nb) return;
+    double* dks = sh.dk[warp];
     const double p = A.bgeom[4L * i], Px = A.bgeom[4L * i + 1], Py = A.bgeom[4L * i + 2], Pz = A.bgeom[4L * i + 3];
     const float Bi = A.bbound[i];
-    // this lane's bra components t = lane + 32 k
-    int tx[NT], ty[NT], tz[NT];
+    // this lane's bra components t = lane + 32 k: their row of the row table, and t_z
+    int trow[NT], tz[NT];
     double jp[NT];
 #pragma unroll
     for (int k = 0; k < NT; ++k) {
         const int t = lane + 32 * k < HB ? lane + 32 * k : 0;
         int N = 0;
         while (nherm_of(N) <= t) ++N;
-        int r = t - nherm_of(N - 1), ii = 0;
+        const int r = N ? t - nherm_of(N - 1) : 0;
+        int ii = 0;
         while ((ii + 1) * (ii + 2) / 2 <= r) ++ii;
         tz[k] = r - ii * (ii + 1) / 2;
-        ty[k] = ii - tz[k];
-        tx[k] = N - ii;
+        trow[k] = (N - ii) * (L + 1) + ii - tz[k];
         jp[k] = 0.0;
     }
     long nq = 0;
@@ -268,12 +314,12 @@ __global__ void __launch_bounds__(kJThreads) k_coulomb_warp(JArgs A)
     for (int j = j0; j < j1; ++j) {
         if (Bi * A.kbound[j] < A.thresp) break;   // kets in bound order
         const double* r = A.krec + (long) j * S;
+        for (int k = lane; k < HK; k += 32) dks[k] = r[4 + g * HK + k];
         const double q = r[0];
         const double X = Px - r[1], Y = Py - r[2], Z = Pz - r[3];
         const double R2 = X * X + Y * Y + Z * Z;
         const double rs = rsqrt(p + q);
         const double rho = p * q * (rs * rs);
-        const double* dk = r + 4 + g * HK;
         ++nq;
         for (int tm = 0; tm < A.nterm; ++tm) {
             const double om = A.omega[tm];
@@ -285,7 +331,7 @@ __global__ void __launch_bounds__(kJThreads) k_coulomb_warp(JArgs A)
             }
             const double rhoe = rho * d2;
             double F[L + 1];
-            boys_eval<L, double>(rhoe * R2, tab, F);
+            boys_eval<L, double>(rhoe * R2, sh.boys, F);
             double a[L + 1];
             const double m2r = -2.0 * rhoe;
             double pw = f;
@@ -294,49 +340,44 @@ __global__ void __launch_bounds__(kJThreads) k_coulomb_warp(JArgs A)
                 a[n] = pw * F[n];
                 pw *= m2r;
             }
-            if (lane == 0) Rb[0] = a[L];
+            // R^(n), n = L .. 0, all orders up to L - n
+            if (lane == 0) sh.R[warp][L & 1][0] = a[L];
             __syncwarp();
-#pragma unroll 1
-            for (int m = L - 1; m >= 0; --m) {
-#pragma unroll 1
-                for (int N = L - m; N >= 1; --N) {
-                    for (int k = lane; k < (N + 1) * (N + 2) / 2; k += 32) {
-                        int ii = 0;
-                        while ((ii + 1) * (ii + 2) / 2 <= k) ++ii;
-                        const int v = k - ii * (ii + 1) / 2, u = ii - v, t = N - ii;
-                        double sv;
-                        if (t > 0) {
-                            sv = X * Rb[herm_pos(t - 1, u, v)];
-                            if (t > 1) sv = fma(double(t - 1), Rb[herm_pos(t - 2, u, v)], sv);
-                        } else if (u > 0) {
-                            sv = Y * Rb[herm_pos(t, u - 1, v)];
-                            if (u > 1) sv = fma(double(u - 1), Rb[herm_pos(t, u - 2, v)], sv);
-                        } else {
-                            sv = Z * Rb[herm_pos(t, u, v - 1)];
-                            if (v > 1) sv = fma(double(v - 1), Rb[herm_pos(t, u, v - 2)], sv);
-                        }
-                        Rb[nherm_of(N - 1) + k] = sv;
-                    }
-                    __syncwarp();
+#pragma unroll
+            for (int n = L - 1; n >= 0; --n) {
+                const double* src = sh.R[warp][(n + 1) & 1];
+                double* dst = sh.R[warp][n & 1];
+                if (lane == 0) dst[0] = a[n];
+#pragma unroll 2
+                for (int k = 1 + lane; k < nherm_of(L - n); k += 32) {
+                    const ushort4 e = sh.step[k];
+                    const int d = e.w & 3;
+                    const double D = d == 0 ? X : (d == 1 ? Y : Z);
+                    dst[e.x] = fma(D, src[e.y], (double) (e.w >> 2) * src[e.z]);
                 }
-                if (lane == 0) Rb[0] = a[m];
                 __syncwarp();
             }
+            const double* Rb = sh.R[warp][0];
+            double sv[NT];
 #pragma unroll
-            for (int k = 0; k < NT; ++k) {
-                if (lane + 32 * k >= HB) break;
-                double sv = jp[k];
-                int uk = 0;
-#pragma unroll 1
-                for (int NK = 0; NK <= LK; ++NK)
-#pragma unroll 1
-                    for (int ik = 0; ik <= NK; ++ik)
-#pragma unroll 1
-                        for (int vk = 0; vk <= ik; ++vk, ++uk)
-                            sv = fma(Rb[herm_pos(tx[k] + NK - ik, ty[k] + ik - vk, tz[k] + vk)], dk[uk], sv);
-                jp[k] = sv;
-            }
-            __syncwarp();   // the table is rebuilt for the next term or ket
+            for (int k = 0; k < NT; ++k) sv[k] = jp[k];
+#pragma unroll
+            for (int ux = 0; ux <= LK; ++ux)
+#pragma unroll
+                for (int uy = 0; uy <= LK - ux; ++uy) {
+                    int at[NT];
+#pragma unroll
+                    for (int k = 0; k < NT; ++k) at[k] = sh.row[trow[k] + ux * (L + 1) + uy] + tz[k];
+#pragma unroll
+                    for (int uz = 0; uz <= LK - ux - uy; ++uz) {
+                        const double dv = dks[herm_pos(ux, uy, uz)];
+#pragma unroll
+                        for (int k = 0; k < NT; ++k) sv[k] = fma(Rb[at[k] + uz], dv, sv[k]);
+                    }
+                }
+#pragma unroll
+            for (int k = 0; k < NT; ++k) jp[k] = sv[k];
+            __syncwarp();   // the tables are rebuilt for the next term or ket
         }
     }
 #pragma unroll
@@ -348,17 +389,35 @@ __global__ void __launch_bounds__(kJThreads) k_coulomb_warp(JArgs A)
 }
 
 template <int LB, int LK>
-void launch_j(Context* ctx, const JArgs& A, int nbra_full, int nket_full)
+void launch_j(Context* ctx, const JArgs& A0, int nbra_full, int nket_full)
 {
     if (nbra_full == 0 || nket_full == 0) return;
     if constexpr (JQ<LB, LK>::loop) {
-        // classes without straight-line code: a bra pair per warp, FP64, a density per CTA z
-        dim3 grid((nbra_full + kJWarpPairs - 1) / kJWarpPairs, (nket_full + A.chunk - 1) / A.chunk, A.ng);
-        k_coulomb_warp<LB, LK><<<grid, kJThreads, 0, ctx->stream>>>(A);
+        // classes without straight-line code: a bra pair per warp, FP64, a density per CTA z.
+        // A CTA holds few pairs, so the default chunk, halved while there are fewer than
+        // four CTAs per multiprocessor, stays larger than the thread-per-pair kernel's
+        // (each CTA makes its tables first)
+        JArgs A = A0;
+        const long tiles = (nbra_full + kJWarpPairs - 1) / kJWarpPairs;
+        if (!A.tuned)
+            for (A.chunk = kJChunk; A.chunk > 16 && tiles * ((nket_full + A.chunk - 1) / A.chunk) < 4L * ctx->nsm;)
+                A.chunk >>= 1;
+        dim3 grid((unsigned) tiles, (nket_full + A.chunk - 1) / A.chunk, A.ng);
+        auto kern = k_coulomb_warp<LB, LK>;
+        constexpr size_t smem = sizeof(JWarpShared<LB, LK>);
+        // the shared-memory opt-in is a per-device function attribute: set it once per device
+        static std::atomic<unsigned long long> devices{0};
+        const unsigned long long bit = 1ull << (ctx->device & 63);
+        if (smem > 48 * 1024 && !(devices.load(std::memory_order_acquire) & bit)) {
+            LSJK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
+            devices.fetch_or(bit, std::memory_order_acq_rel);
+        }
+        kern<<<grid, kJThreads, smem, ctx->stream>>>(A);
         LSJK_CUDA(cudaGetLastError());
         ctx->stats.kernel_launches++;
         return;
     }
+    const JArgs& A = A0;
     // one launch for all densities: CTA z takes NG of them over the same ket
     // records (NG = the class's batch when there are that many, else 1)
     constexpr int NGB = j_batch<LB>();
