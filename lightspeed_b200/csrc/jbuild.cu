@@ -510,6 +510,118 @@ __global__ void k_bra_grad(const int* __restrict__ nbra, const int* __restrict__
     });
 }
 
+// The same for bra classes LB >= 2, a warp per bra pair: lane o (and o + 32, ...) owns the
+// Cartesian component pair (x, y) = (o / N2, o % N2), raises the 1-D coefficient
+// vectors of each direction in registers (as k_herm_to_cart_warp) -- of the value and of
+// the derivatives 2 alpha E^{i+1,j} - i E^{i-1,j} at A and 2 beta E^{i,j+1} - j E^{i,j-1}
+// at B -- and contracts them with the potential. A thread per pair keeps the whole
+// coefficient table in local memory and leaves a small molecule's few pairs on a few
+// warps: (H2O)2/cc-pVTZ, class 6, 940 us.
+template <int LB>
+__global__ void __launch_bounds__(128) k_bra_grad_warp(const int* __restrict__ nbra, const int* __restrict__ p1,
+                                                       const int* __restrict__ p2, const double* __restrict__ geom,
+                                                       BasisView b1, BasisView b2, int symm,
+                                                       const double* __restrict__ vbra, const double* __restrict__ Dc,
+                                                       double scale, double* __restrict__ G)
+{
+    constexpr int H = nherm_of(LB + 1), V = LB + 2;
+    const int lane = threadIdx.x & 31;
+    const long k = ((long) blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (k >= *nbra) return;   // whole warps leave together
+    const int i = p1[k], j = p2[k];
+    const int L1 = b1.L[i], L2 = LB - L1;
+    const int N1 = ncart_of(L1), N2 = ncart_of(L2);
+    const double* g = geom + 4L * k;
+    const double p = g[0];
+    const double A[3] = {b1.x[i], b1.y[i], b1.z[i]};
+    const double B[3] = {b2.x[j], b2.y[j], b2.z[j]};
+    double PA[3], PB[3];
+    double R2 = 0.0;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        PA[d] = g[1 + d] - A[d];
+        PB[d] = g[1 + d] - B[d];
+        R2 += (A[d] - B[d]) * (A[d] - B[d]);
+    }
+    const double e1 = b1.e[i], e2 = b2.e[j];
+    double pre = scale * kTwoPi52 / p * b1.c[i] * b2.c[j] * exp(-e1 * e2 / p * R2);
+    if (symm && i == j) pre *= 0.5;
+    const double h = 0.5 / p;
+    const double* vt = vbra + k * H;
+    const int a1 = b1.cart[i], a2 = b2.cart[j], ld = b2.ncart;
+    struct Ev {
+        double v[V];
+    };
+    // E^{n1,n2}_t of one direction (zero for a negative exponent)
+    auto vec = [h](int n1, int n2, double XA, double XB) {
+        Ev e;
+#pragma unroll
+        for (int t = 0; t < V; ++t) e.v[t] = t == 0 && n1 >= 0 && n2 >= 0 ? 1.0 : 0.0;
+#pragma unroll
+        for (int r = 0; r < LB + 1; ++r) {
+            if (r >= n1 + n2) break;
+            const double X = r < n1 ? XA : XB;
+            Ev n;
+#pragma unroll
+            for (int t = 0; t < V; ++t) {
+                double s = X * e.v[t];
+                if (t > 0) s += h * e.v[t - 1];
+                if (t + 1 < V) s += (t + 1) * e.v[t + 1];
+                n.v[t] = s;
+            }
+            e = n;
+        }
+        return e;
+    };
+    auto comb = [](double a, const Ev& x, int n, const Ev& y) {
+        Ev e;
+#pragma unroll
+        for (int t = 0; t < V; ++t) e.v[t] = a * x.v[t] - n * y.v[t];
+        return e;
+    };
+    double gA[3] = {0.0, 0.0, 0.0}, gB[3] = {0.0, 0.0, 0.0};
+    for (int o = lane; o < N1 * N2; o += 32) {
+        const int x = o / N2, y = o - x * N2;
+        double dxy = Dc[(long) (a1 + x) * ld + a2 + y];
+        if (symm) dxy += Dc[(long) (a2 + y) * ld + a1 + x];
+        const int l[3] = {cart_lx(L1, x), cart_ly(L1, x), cart_lz(L1, x)};
+        const int m[3] = {cart_lx(L2, y), cart_ly(L2, y), cart_lz(L2, y)};
+        const Ev e0 = vec(l[0], m[0], PA[0], PB[0]), e1v = vec(l[1], m[1], PA[1], PB[1]),
+                 e2v = vec(l[2], m[2], PA[2], PB[2]);
+        constexpr HermTab ht = make_herm_tab();
+        // one direction at a time: sum_t D_t^A,B (e e V)_t with the other two directions' products
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const Ev dA = comb(2.0 * e1, vec(l[d] + 1, m[d], PA[d], PB[d]), l[d], vec(l[d] - 1, m[d], PA[d], PB[d]));
+            const Ev dB = comb(2.0 * e2, vec(l[d], m[d] + 1, PA[d], PB[d]), m[d], vec(l[d], m[d] - 1, PA[d], PB[d]));
+            double sa = 0.0, sb = 0.0;
+#pragma unroll
+            for (int t = 0; t < H; ++t) {
+                const int td = d == 0 ? ht.x[t] : (d == 1 ? ht.y[t] : ht.z[t]);
+                const double f = vt[t] * (d == 0 ? e1v.v[ht.y[t]] * e2v.v[ht.z[t]]
+                                                 : (d == 1 ? e0.v[ht.x[t]] * e2v.v[ht.z[t]]
+                                                           : e0.v[ht.x[t]] * e1v.v[ht.y[t]]));
+                sa = fma(dA.v[td], f, sa);
+                sb = fma(dB.v[td], f, sb);
+            }
+            gA[d] = fma(dxy, sa, gA[d]);
+            gB[d] = fma(dxy, sb, gB[d]);
+        }
+    }
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        double sa = gA[d], sb = gB[d];
+        for (int o = 16; o > 0; o >>= 1) {
+            sa += __shfl_xor_sync(0xffffffffu, sa, o);
+            sb += __shfl_xor_sync(0xffffffffu, sb, o);
+        }
+        if (lane == 0) {
+            atomicAdd(&G[3 * b1.atom[i] + d], pre * sa);
+            atomicAdd(&G[3 * b2.atom[j] + d], pre * sb);
+        }
+    }
+}
+
 // Algorithmic FP64/FP32 flops of one J quartet of Hermite class (LB|LK):
 // prefactor/geometry 16, Boys (table 8 FMA + L recursion steps + exp),
 // Hermite recursion (one FMA per R^{(n)}_{tuv}) and the contraction (2 flops
@@ -783,12 +895,21 @@ static void coulomb_grad_bra(Context* ctx, const Ewald& ew, const PairList* pl, 
     DS.n = 1;
     DS.slots = 1;
     const KetSet KS = prepare_kets(ctx, pl, pl, DS, thresp, false);
+    double* vbras[kNHerm] = {};
+    for (int LB = 0; LB < kNHerm; ++LB) {
+        const long nv = (long) pl->jb[LB].n * nherm_of(LB + 1);
+        if (!nv) continue;
+        vbras[LB] = take<double>(ctx, nv);
+        LSJK_CUDA(cudaMemsetAsync(vbras[LB], 0, sizeof(double) * nv, s));
+    }
+    // class kernels go round-robin to the auxiliary streams, as in the J build
+    fork_aux(ctx);
+    int lane = 0;
     for (int LB = 0; LB < kNHerm; ++LB) {
         const JBraClass& jb = pl->jb[LB];
         if (!jb.n) continue;
         const int H1 = nherm_of(LB + 1);
-        double* vbra = take<double>(ctx, (long) jb.n * H1);
-        LSJK_CUDA(cudaMemsetAsync(vbra, 0, sizeof(double) * jb.n * H1, s));
+        double* vbra = vbras[LB];
         for (int LK = 0; LK < kNHerm; ++LK) {
             const JBraClass& jk = pl->jb[LK];
             if (!jk.n) continue;
@@ -820,6 +941,7 @@ static void coulomb_grad_bra(Context* ctx, const Ewald& ew, const PairList* pl, 
                 A.omega[t] = ew.omega[t];
             }
             A.thresp = thresp;
+            OnAux on(ctx, lane++);
             switch (LB + 1) {
             case 1: launch_j_row<1>(ctx, A, LK, jb.n, jk.n); break;
             case 2: launch_j_row<2>(ctx, A, LK, jb.n, jk.n); break;
@@ -831,21 +953,30 @@ static void coulomb_grad_bra(Context* ctx, const Ewald& ew, const PairList* pl, 
             default: throw Error(LSJK_ENOTSUPP, "J gradient: bra Hermite class above 7");
             }
         }
+    }
+    join_aux(ctx);
+    fork_aux(ctx);
+    for (int LB = 0; LB < kNHerm; ++LB) {
+        const JBraClass& jb = pl->jb[LB];
+        if (!jb.n) continue;
         const BasisView v1 = pl->b1->view(), v2 = pl->b2->view();
-        const unsigned gr = nblk(jb.n, 64);
+        const double* vbra = vbras[LB];
+        OnAux on(ctx, lane++);
+        cudaStream_t t = ctx->stream;
         switch (LB) {
-        case 0: k_bra_grad<0><<<gr, 64, 0, s>>>(KS.nbra + LB, jb.p1.p, jb.p2.p, jb.geom.p, v1, v2, pl->symm, vbra, Dbra, scale, G); break;
-        case 1: k_bra_grad<1><<<gr, 64, 0, s>>>(KS.nbra + LB, jb.p1.p, jb.p2.p, jb.geom.p, v1, v2, pl->symm, vbra, Dbra, scale, G); break;
-        case 2: k_bra_grad<2><<<gr, 64, 0, s>>>(KS.nbra + LB, jb.p1.p, jb.p2.p, jb.geom.p, v1, v2, pl->symm, vbra, Dbra, scale, G); break;
-        case 3: k_bra_grad<3><<<gr, 64, 0, s>>>(KS.nbra + LB, jb.p1.p, jb.p2.p, jb.geom.p, v1, v2, pl->symm, vbra, Dbra, scale, G); break;
-        case 4: k_bra_grad<4><<<gr, 64, 0, s>>>(KS.nbra + LB, jb.p1.p, jb.p2.p, jb.geom.p, v1, v2, pl->symm, vbra, Dbra, scale, G); break;
-        case 5: k_bra_grad<5><<<gr, 64, 0, s>>>(KS.nbra + LB, jb.p1.p, jb.p2.p, jb.geom.p, v1, v2, pl->symm, vbra, Dbra, scale, G); break;
-        case 6: k_bra_grad<6><<<gr, 64, 0, s>>>(KS.nbra + LB, jb.p1.p, jb.p2.p, jb.geom.p, v1, v2, pl->symm, vbra, Dbra, scale, G); break;
+        case 0: k_bra_grad<0><<<nblk(jb.n, 64), 64, 0, t>>>(KS.nbra + LB, jb.p1.p, jb.p2.p, jb.geom.p, v1, v2, pl->symm, vbra, Dbra, scale, G); break;
+        case 1: k_bra_grad<1><<<nblk(jb.n, 64), 64, 0, t>>>(KS.nbra + LB, jb.p1.p, jb.p2.p, jb.geom.p, v1, v2, pl->symm, vbra, Dbra, scale, G); break;
+        case 2: k_bra_grad_warp<2><<<nblk(jb.n, 4), 128, 0, t>>>(KS.nbra + LB, jb.p1.p, jb.p2.p, jb.geom.p, v1, v2, pl->symm, vbra, Dbra, scale, G); break;
+        case 3: k_bra_grad_warp<3><<<nblk(jb.n, 4), 128, 0, t>>>(KS.nbra + LB, jb.p1.p, jb.p2.p, jb.geom.p, v1, v2, pl->symm, vbra, Dbra, scale, G); break;
+        case 4: k_bra_grad_warp<4><<<nblk(jb.n, 4), 128, 0, t>>>(KS.nbra + LB, jb.p1.p, jb.p2.p, jb.geom.p, v1, v2, pl->symm, vbra, Dbra, scale, G); break;
+        case 5: k_bra_grad_warp<5><<<nblk(jb.n, 4), 128, 0, t>>>(KS.nbra + LB, jb.p1.p, jb.p2.p, jb.geom.p, v1, v2, pl->symm, vbra, Dbra, scale, G); break;
+        case 6: k_bra_grad_warp<6><<<nblk(jb.n, 4), 128, 0, t>>>(KS.nbra + LB, jb.p1.p, jb.p2.p, jb.geom.p, v1, v2, pl->symm, vbra, Dbra, scale, G); break;
         default: throw Error(LSJK_ENOTSUPP, "J gradient: bra Hermite class above 6");
         }
         LSJK_CUDA(cudaGetLastError());
         ctx->stats.kernel_launches++;
     }
+    join_aux(ctx);
 }
 
 // E = sum D12 (12|34) D34 moves with all four centres: its gradient is the
