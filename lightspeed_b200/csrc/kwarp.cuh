@@ -5,15 +5,22 @@
 // integral tables per lane: 32 lanes' tables no longer fit the SM's L1 and
 // the loop-form quartet runs out of L2. Here the warp shares one set of
 // tables in shared memory and splits each quartet:
-//   * the Rys roots and weights: every lane (the same values);
-//   * per root, lanes 0-2 run the vertical recursion and the transfer to
-//     centre 2 of one direction each; the transfers to centre 4 go one
-//     (direction, a, b) row per lane;
+//   * for a group of roots at a time (all of them but in the largest classes), one
+//     (root, direction) per lane evaluates its root and runs the vertical
+//     recursion, in registers, and the transfer to centre 2, so a quartet pays for
+//     that serial chain once or twice and not once per root;
+//   * per root, the transfers to centre 4 go one (direction, a, b) row per lane;
 //   * the contraction K[i1, i3] += sum_{i2, i4} Ix Iy Iz D[i2, i4] is split
 //     into jobs (i1, i3, a range of i2) over the lanes; each lane keeps its
 //     jobs' sums in registers over the partner-1 entries of a shell segment,
 //     and at the segment's end the parts of an element are added in shared
 //     memory and reach K with one atomic per element.
+// Bound by the latency of these phases and by shared-memory reads in the
+// contraction, so registers are held to 128 (16 warps per multiprocessor; 168
+// without the bound: 12.8 against 12.4 ms for the build below). With lanes 0-2 running
+// every root's recursion in shared memory, one root after another, and component
+// indices decoded in the contraction, this kernel took 19.2 of the 33.6 ms of class
+// kernels in the (H2O)4/cc-pVTZ J+K build; now 10.8 (build 15.6 -> 12.4 ms).
 // Work order and screens are those of k_exchange (a (prim2, prim4) task per
 // warp, here split into stripes of its partners 3; partners 3 outer, partners 1
 // of each partner 3 in segment order), FP64 only, one density per task and
@@ -54,19 +61,23 @@ struct KWarpShape {
     static constexpr int NO = N1 * N3;                                      // output elements
     static constexpr int P = NO >= 32 ? 1 : (N2 < 32 / NO ? N2 : 32 / NO);   // i2 parts per element
     static constexpr int NJOB = NO * P, NJL = (NJOB + 31) / 32;             // jobs, jobs per lane
+    static constexpr int NR = (L1 + L2 + L3 + L4) / 2 + 1;
+    // roots per group: as many as keep the group's tables within 1600 doubles per warp
+    static constexpr int SH = 3 * S2 * (LA + 1) * (LC + 1);
+    static constexpr int RG = NR * SH <= 1600 ? NR : (1600 / SH > 1 ? 1600 / SH : 1);
 };
 
 template <int L1, int L2, int L3, int L4>
 struct KWarpTab {
     using S = KWarpShape<L1, L2, L3, L4>;
     double G[3][S::SG];                            // 1-D integrals of the current root
-    double H[3][L2 + 1][S::LA + 1][S::LC + 1];     // after the transfer to centre 2
+    double H[S::RG][3][L2 + 1][S::LA + 1][S::LC + 1];   // a group's integrals at centre 2
     double D[S::N2 * S::N4];                       // the task's D24 block
     double red[S::NJOB];                           // job sums at a segment flush
 };
 
 template <int L1, int L2, int L3, int L4>
-__global__ void __launch_bounds__(kKThreads) k_exchange_warp(const __grid_constant__ KArgs A)
+__global__ void __launch_bounds__(kKThreads, 4) k_exchange_warp(const __grid_constant__ KArgs A)
 {
     using Sh = KWarpShape<L1, L2, L3, L4>;
     constexpr int NR = (L1 + L2 + L3 + L4) / 2 + 1;
@@ -85,17 +96,27 @@ __global__ void __launch_bounds__(kKThreads) k_exchange_warp(const __grid_consta
     const double* asym_w = static_cast<const double*>(A.asym_w);
     const float thre12 = A.sc->thre12, thre34 = A.sc->thre34;
     const double thr_lo = (double) A.thr_lo, thr_hi = (double) A.thr_hi;
+    // offsets of shell 2's components in the tables of the three directions
+    __shared__ int off2[N2][3];
+    for (int k = threadIdx.x; k < N2; k += kKThreads) {
+        off2[k][0] = cart_lx(L2, k) * S3 * S4;
+        off2[k][1] = cart_ly(L2, k) * S3 * S4;
+        off2[k][2] = cart_lz(L2, k) * S3 * S4;
+    }
+    __syncthreads();
+    const int rl = lane / 3, dl = lane % 3;   // this lane's root of a group, and direction
 
     // this lane's jobs: element o = job / P (i1 = o / N3, i3 = o % N3), i2 range part = job % P
-    int jx[NJL][2], jy[NJL][2], jz[NJL][2];   // Cartesian exponents of shells 1 and 3
+    int jx[NJL], jy[NJL], jz[NJL];   // table offsets of its components of shells 1 and 3
     int j2lo[NJL], j2hi[NJL];
 #pragma unroll
     for (int k = 0; k < NJL; ++k) {
         const int job = lane + 32 * k;
         const int o = job < NJOB ? job / P : 0, part = job < NJOB ? job % P : 0;
         const int i1 = o / N3, i3 = o % N3;
-        jx[k][0] = cart_lx(L1, i1); jy[k][0] = cart_ly(L1, i1); jz[k][0] = cart_lz(L1, i1);
-        jx[k][1] = cart_lx(L3, i3); jy[k][1] = cart_ly(L3, i3); jz[k][1] = cart_lz(L3, i3);
+        jx[k] = (cart_lx(L1, i1) * S2 * S3 + cart_lx(L3, i3)) * S4;
+        jy[k] = (cart_ly(L1, i1) * S2 * S3 + cart_ly(L3, i3)) * S4;
+        jz[k] = (cart_lz(L1, i1) * S2 * S3 + cart_lz(L3, i3)) * S4;
         j2lo[k] = job < NJOB ? part * N2 / P : 0;
         j2hi[k] = job < NJOB ? (part + 1) * N2 / P : 0;
     }
@@ -159,10 +180,17 @@ __global__ void __launch_bounds__(kKThreads) k_exchange_warp(const __grid_consta
                 }
                 any = false;
             };
+            // the next entry's bound and segment are loaded one iteration ahead
+            float bn = A.b12[s12];
+            int sn = A.seg12[s12];
             for (int j = 0; j < n12; ++j) {
                 const int e = s12 + j;
-                const float b12 = A.b12[e];
-                const int sg = A.seg12[e];
+                const float b12 = bn;
+                const int sg = sn;
+                if (j + 1 < n12) {
+                    bn = A.b12[e + 1];
+                    sn = A.seg12[e + 1];
+                }
                 if (ns1 > 1 && sg % ns1 != stripe1) continue;   // another unit's segment
                 const float est = b12 * b34;
                 const bool can = b12 >= thre12 && est >= tlo;
@@ -182,7 +210,6 @@ __global__ void __launch_bounds__(kKThreads) k_exchange_warp(const __grid_consta
                 const double AB[3] = {A.d12.ax[e], A.d12.ay[e], A.d12.az[e]};
                 const double PQ[3] = {ex + Sx, ey + Sy, ez + Sz};
                 const double PA[3] = {ex - AB[0], ey - AB[1], ez - AB[2]};
-                const double CD[3] = {Cx, Cy, Cz};
                 const double RR = PQ[0] * PQ[0] + PQ[1] * PQ[1] + PQ[2] * PQ[2];
                 const double rs = rsqrt(p + q);
                 const double ipq = rs * rs;
@@ -195,75 +222,93 @@ __global__ void __launch_bounds__(kKThreads) k_exchange_warp(const __grid_consta
                         d2 = w2 / (rho + w2);
                         f *= sqrt(d2);
                     }
-                    double t2[NR], w[NR];
-                    rys_eval<NR, double>(rho * d2 * RR, tab, A.nbin, A.tmax, asym_t, asym_w, t2, w);
+                    const double T = rho * d2 * RR;
 #pragma unroll 1
-                    for (int r = 0; r < NR; ++r) {
-                        const double u = t2[r] * d2 * ipq;
-                        const double qu = q * u, pu = p * u;
-                        const double b00 = 0.5 * u, b10 = 0.5 * ip * (1.0 - qu), b01 = 0.5 * iq * (1.0 - pu);
-                        if (lane < 3) {
-                            // 2-D integrals I(a, c) of direction `lane`, then moved to centre 2
-                            const int d = lane;
-                            const double c00 = PA[d] - qu * PQ[d], d00 = QC[d] + pu * PQ[d], ab = AB[d];
-                            auto& H = S.H[d];
-                            H[0][0][0] = d == 2 ? f * w[r] : 1.0;
+                    for (int r0 = 0; r0 < NR; r0 += Sh::RG) {
+                        if (lane < 3 * Sh::RG && r0 + rl < NR) {
+                            // 2-D integrals I(a, c) of root r0 + rl in direction dl
+                            double t2, w;
+                            rys_root(T, tab, NR, r0 + rl, A.nbin, A.tmax, asym_t, asym_w, t2, w);
+                            const double u = t2 * d2 * ipq, qu = q * u, pu = p * u;
+                            const double b00 = 0.5 * u, b10 = 0.5 * ip * (1.0 - qu), b01 = 0.5 * iq * (1.0 - pu);
+                            const double PQd = dl == 0 ? PQ[0] : (dl == 1 ? PQ[1] : PQ[2]);
+                            const double ABd = dl == 0 ? AB[0] : (dl == 1 ? AB[1] : AB[2]);
+                            const double c00 = (dl == 0 ? PA[0] : (dl == 1 ? PA[1] : PA[2])) - qu * PQd;
+                            const double d00 = (dl == 0 ? QC[0] : (dl == 1 ? QC[1] : QC[2])) + pu * PQd;
+                            double I[LA + 1][LC + 1];
+                            I[0][0] = dl == 2 ? f * w : 1.0;
+#pragma unroll
                             for (int a = 1; a <= LA; ++a) {
-                                double s = c00 * H[0][a - 1][0];
-                                if (a > 1) s = fma((a - 1) * b10, H[0][a - 2][0], s);
-                                H[0][a][0] = s;
+                                double s = c00 * I[a - 1][0];
+                                if (a > 1) s = fma((a - 1) * b10, I[a - 2][0], s);
+                                I[a][0] = s;
                             }
+#pragma unroll
                             for (int c = 1; c <= LC; ++c)
+#pragma unroll
                                 for (int a = 0; a <= LA; ++a) {
-                                    double s = d00 * H[0][a][c - 1];
-                                    if (c > 1) s = fma((c - 1) * b01, H[0][a][c - 2], s);
-                                    if (a > 0) s = fma(a * b00, H[0][a - 1][c - 1], s);
-                                    H[0][a][c] = s;
+                                    double s = d00 * I[a][c - 1];
+                                    if (c > 1) s = fma((c - 1) * b01, I[a][c - 2], s);
+                                    if (a > 0) s = fma(a * b00, I[a - 1][c - 1], s);
+                                    I[a][c] = s;
                                 }
-                            for (int b = 1; b <= L2; ++b)
-                                for (int a = 0; a <= LA - b; ++a)
-                                    for (int c = 0; c <= LC; ++c) H[b][a][c] = fma(ab, H[b - 1][a][c], H[b - 1][a + 1][c]);
-                        }
-                        __syncwarp();
-                        // to centre 4: one (direction, a, b) row per lane
-                        for (int row = lane; row < 3 * (L1 + 1) * S2; row += 32) {
-                            const int d = row / ((L1 + 1) * S2), a = (row / S2) % (L1 + 1), b = row % S2;
-                            double Tr[L4 + 1][LC + 1];
+                            // moved to centre 2, in place
+                            auto& H = S.H[rl][dl];
 #pragma unroll
-                            for (int c = 0; c <= LC; ++c) Tr[0][c] = S.H[d][b][a][c];
+                            for (int b = 0; b <= L2; ++b) {
 #pragma unroll
-                            for (int e4 = 1; e4 <= L4; ++e4)
+                                for (int a = 0; a <= LA - b && a <= L1; ++a)
 #pragma unroll
-                                for (int c = 0; c <= LC - e4; ++c) Tr[e4][c] = fma(CD[d], Tr[e4 - 1][c], Tr[e4 - 1][c + 1]);
+                                    for (int c = 0; c <= LC; ++c) H[b][a][c] = I[a][c];
 #pragma unroll
-                            for (int c = 0; c <= L3; ++c)
+                                for (int a = 0; a + 1 <= LA - b; ++a)
 #pragma unroll
-                                for (int e4 = 0; e4 <= L4; ++e4) S.G[d][((a * S2 + b) * S3 + c) * S4 + e4] = Tr[e4][c];
-                        }
-                        __syncwarp();
-                        // the contraction jobs of this lane
-#pragma unroll
-                        for (int k = 0; k < NJL; ++k) {
-                            double s = acc[k];
-                            const int x1 = jx[k][0], y1 = jy[k][0], z1 = jz[k][0];
-                            const int x3 = jx[k][1], y3 = jy[k][1], z3 = jz[k][1];
-#pragma unroll 1
-                            for (int i2c = j2lo[k]; i2c < j2hi[k]; ++i2c) {
-                                const int x2 = cart_lx(L2, i2c), y2 = cart_ly(L2, i2c), z2 = cart_lz(L2, i2c);
-                                const double* gx = &S.G[0][((x1 * S2 + x2) * S3 + x3) * S4];
-                                const double* gy = &S.G[1][((y1 * S2 + y2) * S3 + y3) * S4];
-                                const double* gz = &S.G[2][((z1 * S2 + z2) * S3 + z3) * S4];
-                                const double* Drow = &S.D[i2c * N4];
-                                int i4 = 0;
-#pragma unroll
-                                for (int j4 = 0; j4 <= L4; ++j4)
-#pragma unroll
-                                    for (int z4 = 0; z4 <= j4; ++z4, ++i4)
-                                        s = fma(gx[L4 - j4] * gy[j4 - z4] * gz[z4], Drow[i4], s);
+                                    for (int c = 0; c <= LC; ++c) I[a][c] = fma(ABd, I[a][c], I[a + 1][c]);
                             }
-                            acc[k] = s;
                         }
-                        __syncwarp();   // the tables are rewritten by the next root
+#pragma unroll 1
+                        for (int r = 0; r < Sh::RG && r0 + r < NR; ++r) {
+                            __syncwarp();
+                            // to centre 4: one (direction, a, b) row per lane
+                            for (int row = lane; row < 3 * (L1 + 1) * S2; row += 32) {
+                                const int d = row / ((L1 + 1) * S2), a = (row / S2) % (L1 + 1), b = row % S2;
+                                const double CDd = d == 0 ? Cx : (d == 1 ? Cy : Cz);
+                                double Tr[L4 + 1][LC + 1];
+#pragma unroll
+                                for (int c = 0; c <= LC; ++c) Tr[0][c] = S.H[r][d][b][a][c];
+#pragma unroll
+                                for (int e4 = 1; e4 <= L4; ++e4)
+#pragma unroll
+                                    for (int c = 0; c <= LC - e4; ++c)
+                                        Tr[e4][c] = fma(CDd, Tr[e4 - 1][c], Tr[e4 - 1][c + 1]);
+#pragma unroll
+                                for (int c = 0; c <= L3; ++c)
+#pragma unroll
+                                    for (int e4 = 0; e4 <= L4; ++e4)
+                                        S.G[d][((a * S2 + b) * S3 + c) * S4 + e4] = Tr[e4][c];
+                            }
+                            __syncwarp();
+                            // the contraction jobs of this lane
+#pragma unroll
+                            for (int k = 0; k < NJL; ++k) {
+                                double s = acc[k];
+#pragma unroll 1
+                                for (int i2c = j2lo[k]; i2c < j2hi[k]; ++i2c) {
+                                    const double* gx = &S.G[0][jx[k] + off2[i2c][0]];
+                                    const double* gy = &S.G[1][jy[k] + off2[i2c][1]];
+                                    const double* gz = &S.G[2][jz[k] + off2[i2c][2]];
+                                    const double* Drow = &S.D[i2c * N4];
+                                    int i4 = 0;
+#pragma unroll
+                                    for (int j4 = 0; j4 <= L4; ++j4)
+#pragma unroll
+                                        for (int z4 = 0; z4 <= j4; ++z4, ++i4)
+                                            s = fma(gx[L4 - j4] * gy[j4 - z4] * gz[z4], Drow[i4], s);
+                                }
+                                acc[k] = s;
+                            }
+                            __syncwarp();   // the tables are rewritten by the next root
+                        }
                     }
                 }
             }
