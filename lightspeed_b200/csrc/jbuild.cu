@@ -769,7 +769,7 @@ void coulomb_build(Context* ctx, const Ewald& ew, const PairList* pl12, const Pa
     // class kernels go round-robin to the auxiliary streams (not while the
     // autotuner times them one by one)
     const bool par = !ctx->tuning;
-    if (par) fork_aux(ctx);
+    if (par) fork_aux(ctx, std::max(pl12->npair, pl34->npair));
     int lane = 0;
     for (int LB = 0; LB < kNHerm; ++LB) {
         const JBraClass& jb = pl12->jb[LB];
@@ -903,7 +903,7 @@ static void coulomb_grad_bra(Context* ctx, const Ewald& ew, const PairList* pl, 
         LSJK_CUDA(cudaMemsetAsync(vbras[LB], 0, sizeof(double) * nv, s));
     }
     // class kernels go round-robin to the auxiliary streams, as in the J build
-    fork_aux(ctx);
+    fork_aux(ctx, pl->npair);
     int lane = 0;
     for (int LB = 0; LB < kNHerm; ++LB) {
         const JBraClass& jb = pl->jb[LB];
@@ -955,7 +955,7 @@ static void coulomb_grad_bra(Context* ctx, const Ewald& ew, const PairList* pl, 
         }
     }
     join_aux(ctx);
-    fork_aux(ctx);
+    fork_aux(ctx, pl->npair);
     for (int LB = 0; LB < kNHerm; ++LB) {
         const JBraClass& jb = pl->jb[LB];
         if (!jb.n) continue;

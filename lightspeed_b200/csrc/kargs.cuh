@@ -71,17 +71,15 @@ struct KArgs {
     const void* rys;          // table block of this rule, in the pass precision
     const void* asym_t;
     const void* asym_w;
-    // FP64 table block and asymptotic nodes of this rule in global memory: the
-    // FP32 pass evaluates the roots and weights in FP64 from the last table bin on
-    const double* rys64g;
-    const double* asym64_t;
-    const double* asym64_w;
     int nbin;
     double tmax;
     int* status;
     unsigned long long* qcount;
     int nterm;
     double alpha[4], omega[4];
+    float alphaf[4];             // alpha in FP32
+    int bare;                    // bit tm: term tm is bare 1/r (omega = -1)
+    int split;                   // k_exchange: partner-1 stripes per task, at most
     int stripes;                 // k_exchange_warp: partner-3 stripes per task (work units per task)
     int split_hi;                // this is the FP64 pass of a mixed build (estimate >= thredp only)
 };

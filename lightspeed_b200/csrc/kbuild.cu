@@ -326,12 +326,15 @@ void exchange_build(Context* ctx, const Ewald& ew, const PairList* pl12, const P
     // class kernels go round-robin to the auxiliary streams (not while the
     // autotuner times them one by one)
     const bool par = !ctx->tuning;
-    if (par) fork_aux(ctx);
+    if (par) fork_aux(ctx, std::max(pl12->npair, pl34->npair));
     int lane = 0;
-    for (int L1 = 0; L1 < kNL; ++L1)
-        for (int L2 = 0; L2 < kNL; ++L2)
-            for (int L3 = 0; L3 < kNL; ++L3)
-                for (int L4 = 0; L4 < kNL; ++L4) {
+    // average partner-1 row of class L1: the entries' share of that shell's primitives
+    const double rows12 = (double) pl12->kdat.nent / ((double) pl12->b1->nprim * b2->nprim);
+    // heaviest quartets first: their tails overlap the lighter classes
+    for (int L1 = kNL - 1; L1 >= 0; --L1)
+        for (int L2 = kNL - 1; L2 >= 0; --L2)
+            for (int L3 = kNL - 1; L3 >= 0; --L3)
+                for (int L4 = kNL - 1; L4 >= 0; --L4) {
                     int c = combo_index(L1, L2, L3, L4);
                     long cap = off[c + 1] - off[c];
                     if (!cap) continue;
@@ -377,6 +380,7 @@ void exchange_build(Context* ctx, const Ewald& ew, const PairList* pl12, const P
                     A.flip = flip_ok ? 1 : 0;
                     A.gc = (pl12->b1->is_twin || pl34->b1->is_twin) ? 1 : 0;
                     A.sc = sc;
+                    A.split = (int) std::max(1.0, std::min(32.0, rows12 * cnt1[L1] / 2.0));
                     A.nbin = kRysNbin[NR];
                     A.tmax = kRysTmax[NR];
                     A.status = ctx->status.p;
@@ -384,6 +388,8 @@ void exchange_build(Context* ctx, const Ewald& ew, const PairList* pl12, const P
                     for (int t = 0; t < A.nterm; ++t) {
                         A.alpha[t] = ew.alpha[t];
                         A.omega[t] = ew.omega[t];
+                        A.alphaf[t] = (float) ew.alpha[t];
+                        if (ew.omega[t] == -1.0) A.bare |= 1 << t;
                     }
                     const float inf = __builtin_huge_valf();
                     // classes above the straight-line quartet code (an f shell) run in FP64 only:
@@ -402,9 +408,6 @@ void exchange_build(Context* ctx, const Ewald& ew, const PairList* pl12, const P
                     A.rys = ctx->rys64.p + kRysOffset[NR];
                     A.asym_t = ctx->rys_asym64.p + NR * LSJK_RYS_NMAX;
                     A.asym_w = ctx->rys_asym64.p + (LSJK_RYS_NMAX + 1) * LSJK_RYS_NMAX + NR * LSJK_RYS_NMAX;
-                    A.rys64g = ctx->rys64.p + kRysOffset[NR];
-                    A.asym64_t = ctx->rys_asym64.p + NR * LSJK_RYS_NMAX;
-                    A.asym64_w = ctx->rys_asym64.p + (LSJK_RYS_NMAX + 1) * LSJK_RYS_NMAX + NR * LSJK_RYS_NMAX;
                     A.qcount = qcnt + c;
                     auto tune = [&](const KArgs& X, bool fp32) {
                         // autotuner: time candidate grid sizes on scratch outputs
@@ -604,7 +607,7 @@ void exchange_grad_symm(Context* ctx, const Ewald& ew, const PairList* pl, const
         off[L1][L2][side] = (int) pl->cls_off[c];
         cnt[L1][L2][side] = (int) (pl->cls_off[c + 1] - pl->cls_off[c]);
     }
-    fork_aux(ctx);
+    fork_aux(ctx, pl->npair);
     int lane = 0;
     // heaviest classes first, so their tails overlap the lighter ones
     for (int L1 = kNL - 1; L1 >= 0; --L1)

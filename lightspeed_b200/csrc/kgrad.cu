@@ -113,7 +113,7 @@ __device__ void kgrad_quartet(const KGradArgs& A, double alpha, double beta, dou
             f *= sqrt(d2);
         }
         double t2[NR], w[NR];
-        rys_eval<NR, double>(rho * d2 * RR, A.rys, A.nbin, A.tmax, A.asym_t, A.asym_w, t2, w);
+        rys_eval<NR, double>(rho * d2 * RR, A.rys, A.nbin, A.tmax, A.nbin / A.tmax, A.asym_t, A.asym_w, t2, w);
 #pragma unroll (UR)
         for (int r = 0; r < NR; ++r) {
             const double u = t2[r] * d2 * ipq;
@@ -386,7 +386,7 @@ __device__ void kgrad_quartet_warp(const KGradArgs& A, KGradWarpTables<L1, L2, L
             f *= sqrt(d2);
         }
         double t2[NR], w[NR];
-        rys_eval<NR, double>(rho * d2 * RR, A.rys, A.nbin, A.tmax, A.asym_t, A.asym_w, t2, w);
+        rys_eval<NR, double>(rho * d2 * RR, A.rys, A.nbin, A.tmax, A.nbin / A.tmax, A.asym_t, A.asym_w, t2, w);
 #pragma unroll 1
         for (int r = 0; r < NR; ++r) {
             const double u = t2[r] * d2 * ipq;

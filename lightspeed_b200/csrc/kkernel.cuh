@@ -61,13 +61,21 @@ struct alignas(16) KEnt {
 // has few tasks per warp, so the queue still balances the load).
 constexpr int kKGrab = 16;
 
+// Work units per warp a class is cut into when it has fewer tasks: a task walks its
+// partner-1 row serially for every 32 partners 3, so with one task per warp or less a
+// class takes as long as its longest rows ((p s|p s) of C10H22: 9% of the warps active
+// on average) and a small molecule's classes leave most of the GPU idle. The rows are
+// cut into up to KArgs::split stripes of two entries or more (a stripe repeats the
+// task's header, D24 loads and segment flush).
+constexpr int kKUnitsPerWarp = 2;
+
 // Everything a task needs before its partner rows, prepared by one lane per
 // task of a grab (the loads of all the grab's tasks overlap) and read by the
-// warp as shared-memory broadcasts (64 bytes).
+// warp as shared-memory broadcasts (80 bytes).
 struct alignas(16) KHdr {
     double dRx, dRy, dRz;   // R2 - R4 (pair data are relative to these centres)
-    int s12, n12, s34, n34; // K-invert rows of prim2 (partners 1) and prim4 (partners 3; n34: the
-                            // prefix of the row that can pass the screens)
+    int s12, k1a, k1b;      // K-invert row of prim2 and this unit's stripe [k1a, k1b) of its partners 1
+    int s34, n34;           // row of prim4 (partners 3; n34: the prefix that can pass the screens)
     int c2, c4;             // Cartesian offsets of prim2 and prim4
     float tlo, thi;         // float thresholds on bound12 * bound34 for this task's max|D24|
     float b12max;           // largest bound of the partner-1 row
@@ -135,7 +143,7 @@ __host__ __device__ constexpr int k_batch()
 // 1-D integrals are shared by the densities (the NG inlined contractions see
 // identical integral inputs).
 template <int L1, int L2, int L3, int L4, typename R, int NG>
-__device__ __forceinline__ void k_quartet(const KArgs& A, const R* __restrict__ tab, R tmax,
+__device__ __forceinline__ void k_quartet(const KArgs& A, const R* __restrict__ tab, R tmax, R tswitch, R bscale,
                                           const R* __restrict__ asym_t, const R* __restrict__ asym_w,
                                           const KEnt<R>& e, R kab34, R q, R iq, R Sx, R Sy, R Sz, R QCx,
                                           R QCy, R QCz, R Cx, R Cy, R Cz, const R (*Dblk)[ncart_of(L2) * ncart_of(L4)],
@@ -154,8 +162,9 @@ __device__ __forceinline__ void k_quartet(const KArgs& A, const R* __restrict__ 
     // kab fields hold K_ab / p per pair
     const R pref = (R) kTwoPi52K * (e.kab * kab34) * rs;
     for (int tm = 0; tm < A.nterm; ++tm) {
-        R d2 = R(1), f = (R) A.alpha[tm] * pref;
-        if (A.omega[tm] != -1.0) {
+        const R al = [&] { if constexpr (sizeof(R) == 4) return A.alphaf[tm]; else return A.alpha[tm]; }();
+        R d2 = R(1), f = al * pref;
+        if (!(A.bare >> tm & 1)) {
             const R w2 = (R) (A.omega[tm] * A.omega[tm]);
             d2 = w2 / (rho + w2);
             f *= sqrt(d2);
@@ -164,22 +173,15 @@ __device__ __forceinline__ void k_quartet(const KArgs& A, const R* __restrict__ 
         if constexpr (sizeof(R) == 4) {
             // FP32 pass: from the last table bin on (the bin next to the switch to the
             // asymptotic form, and the asymptotic region) the roots and weights are the
-            // FP64 asymptotic form t = s / sqrt(T), w = h / sqrt(T), which over the last
-            // bin already agrees with the exact rule to ~1e-13 relative
+            // asymptotic form t = s / sqrt(T), w = h / sqrt(T) to better than FP32, which
+            // over the last bin already agrees with the exact rule to ~1e-13 relative
             const R T = rho * d2 * RR;
-            if (T < tmax - tmax / (R) A.nbin) {
-                rys_eval<NR, R>(T, tab, A.nbin, tmax, asym_t, asym_w, t2, w);
-            } else {
-                const double r = rsqrt_f64_newton((double) rho * (double) d2 * (double) RR);
-#pragma unroll
-                for (int i = 0; i < NR; ++i) {
-                    const double t = c_rys_asym_t[NR * LSJK_RYS_NMAX + i] * r;
-                    t2[i] = (R) (t * t);
-                    w[i] = (R) (c_rys_asym_w[NR * LSJK_RYS_NMAX + i] * r);
-                }
-            }
+            if (T < tswitch)
+                rys_eval<NR, R>(T, tab, A.nbin, tmax, bscale, asym_t, asym_w, t2, w);
+            else
+                rys_asym_pairs<NR>(rho, d2, RR, t2, w);
         } else {
-            rys_eval<NR, R>(rho * d2 * RR, tab, A.nbin, tmax, asym_t, asym_w, t2, w);
+            rys_eval<NR, R>(rho * d2 * RR, tab, A.nbin, tmax, bscale, asym_t, asym_w, t2, w);
         }
         auto root = [&](int r) {
             const R u = t2[r] * d2 * ipq;
@@ -192,22 +194,18 @@ __device__ __forceinline__ void k_quartet(const KArgs& A, const R* __restrict__ 
                 kq_dispatch<L1, L2, L3, L4>(c00x, c00y, c00z, d00x, d00y, d00z, b00, b10, b01, e.ax, e.ay, e.az,
                                             Cx, Cy, Cz, f * w[r], Dblk[g], acc[g]);
         };
-        if constexpr (sizeof(R) == 4) {
-            // FP32: roots one after another (fewer live registers, more resident warps);
-            // the root in use is always slot 0 and the rest shift down, so the
-            // arrays keep static indices and stay in registers
+        // roots one after another (fewer live registers, more resident warps in FP32; one copy
+        // of the root's code instead of up to five in FP64, which a small molecule's kernels
+        // otherwise spend their time fetching): the root in use is always slot 0 and the rest
+        // shift down, so the arrays keep static indices and stay in registers
 #pragma unroll 1
-            for (int r = 0; r < NR; ++r) {
-                root(0);
+        for (int r = 0; r < NR; ++r) {
+            root(0);
 #pragma unroll
-                for (int i = 0; i + 1 < NR; ++i) {
-                    t2[i] = t2[i + 1];
-                    w[i] = w[i + 1];
-                }
+            for (int i = 0; i + 1 < NR; ++i) {
+                t2[i] = t2[i + 1];
+                w[i] = w[i + 1];
             }
-        } else {
-#pragma unroll
-            for (int r = 0; r < NR; ++r) root(r);
         }
     }
 }
@@ -228,7 +226,10 @@ __global__ void __launch_bounds__(kKThreads) k_exchange(const __grid_constant__ 
     __shared__ KEnt<R> ring_all[kKWarps][2][32];
     __shared__ KHdr hdr_all[kKWarps][kKGrab];
     const int ntask1 = *A.ntask;
-    const int ntask = ntask1 * A.nsub;   // the task list once per density sub-slot
+    const int ntask_all = ntask1 * A.nsub;   // the task list once per density sub-slot
+    // and once per partner-1 stripe
+    const int nstripe = max(1, min(A.split, kKUnitsPerWarp * (int) gridDim.x * kKWarps / max(1, ntask_all)));
+    const int ntask = ntask_all * nstripe;
     // the grid is sized for the class's task capacity; CTAs whose warps cannot
     // get a task leave before staging the quadrature table
     if ((long) blockIdx.x * kKWarps >= ntask) return;
@@ -236,7 +237,8 @@ __global__ void __launch_bounds__(kKThreads) k_exchange(const __grid_constant__ 
     if (!stage_bulk(tab, A.rys, bytes, &mbar, A.status)) return;
     const R* asym_t = static_cast<const R*>(A.asym_t);
     const R* asym_w = static_cast<const R*>(A.asym_w);
-    const R tmax = (R) A.tmax;
+    const R tmax = (R) A.tmax, bscale = (R) A.nbin / tmax;   // (bins per unit of T)
+    const R tswitch = tmax - tmax / (R) A.nbin;                     // start of the last table bin
 
     const KRows<R> d12 = [&] { if constexpr (FP64) return A.d12; else return A.f12; }();
     const KRows<R> d34 = [&] { if constexpr (FP64) return A.d34; else return A.f34; }();
@@ -261,8 +263,9 @@ __global__ void __launch_bounds__(kKThreads) k_exchange(const __grid_constant__ 
         __syncwarp();   // the previous grab's headers have been read
         if (lane < nt) {
             const int tv = t0 + lane;
-            const int sub = tv / ntask1;
-            const KTask T = A.tasks[tv - sub * ntask1];
+            const int stripe = tv / ntask_all, ts = tv - stripe * ntask_all;
+            const int sub = ts / ntask1;
+            const KTask T = A.tasks[ts - sub * ntask1];
             const int i2 = T.i2, i4 = T.i4;
             KHdr h;
             h.dbase = T.grp * kKBatch + sub * NG;
@@ -271,7 +274,9 @@ __global__ void __launch_bounds__(kKThreads) k_exchange(const __grid_constant__ 
             h.dRy = A.b2.y[i2] - A.b4.y[i4];
             h.dRz = A.b2.z[i2] - A.b4.z[i4];
             h.s12 = A.r12s[i2];
-            h.n12 = A.r12l[i2];
+            const int n12 = A.r12l[i2];
+            h.k1a = n12 * stripe / nstripe;
+            h.k1b = n12 * (stripe + 1) / nstripe;
             h.s34 = A.r34s[i4];
             h.n34 = A.r34l[i4];
             h.c2 = A.b2.cart[i2];
@@ -290,7 +295,8 @@ __global__ void __launch_bounds__(kKThreads) k_exchange(const __grid_constant__ 
                     const float b = A.b34[h.s34 + mid];
                     if (b >= thre34 && h.b12max * b >= h.tlo) lo = mid + 1; else hi = mid;
                 }
-                h.n34 = h.dn > 0 ? lo : 0;   // a sub-slot past the group's densities: no work
+                // (a sub-slot past the group's densities, or an empty stripe: no work)
+                h.n34 = h.dn > 0 && h.k1a < h.k1b ? lo : 0;
             }
             // symmetric D24 (A.flip): the transposed contribution of a task with i2 != i4 is
             // not written here; the build adds K13 to its transpose afterwards, and tasks with
@@ -308,13 +314,14 @@ __global__ void __launch_bounds__(kKThreads) k_exchange(const __grid_constant__ 
         for (;;) {
             while (pos < nt && hdr[pos].n34 == 0) ++pos;
             if (pos >= nt) break;
-            const int s12 = hdr[pos].s12, n12 = hdr[pos].n12, c2 = hdr[pos].c2;
+            const int s12 = hdr[pos].s12, k1a = hdr[pos].k1a, n12 = hdr[pos].k1b, c2 = hdr[pos].c2;
             // the pack's densities (its tasks share prim2 and the density sub-slot)
             const int dbase = hdr[pos].dbase, dn = hdr[pos].dn;
             int my_task = -1, my_k = 0;
             {
                 int filled = 0, at = pos, k0 = koff;
-                while (filled < 32 && at < nt && hdr[at].s12 == s12 && hdr[at].dbase == dbase) {
+                while (filled < 32 && at < nt && hdr[at].s12 == s12 && hdr[at].k1a == k1a &&
+                       hdr[at].dbase == dbase) {
                     const int n = hdr[at].n34;
                     const int len = min(n - k0, 32 - filled);
                     if (lane >= filled && lane < filled + len) {
@@ -373,8 +380,6 @@ __global__ void __launch_bounds__(kKThreads) k_exchange(const __grid_constant__ 
                         w31 = A.w1_34[k3];
                     }
                 }
-                // (every lane of a pack passes thre34 and the row's first partner 1)
-                const bool v3 = in3;
                 const R QCx = Qx - Cx, QCy = Qy - Cy, QCz = Qz - Cz;
                 // ket side of PQ: (Q - R4) with the task's centre shift folded in
                 const R Sx = dRx - Qx, Sy = dRy - Qy, Sz = dRz - Qz;
@@ -391,6 +396,11 @@ __global__ void __launch_bounds__(kKThreads) k_exchange(const __grid_constant__ 
                 }
                 bool any = false;
                 int prev_seg = -1, prev_c1 = 0, prev_c1b = -1;
+                // a stripe may start inside a shell segment, whose largest bound came before it:
+                // its first entry is then not taken for the segment's
+                int last_seg = k1a > 0 ? A.seg12[s12 + k1a - 1] : -1;
+                const float rmax = __int_as_float((int) __reduce_max_sync(
+                    0xffffffffu, (unsigned) __float_as_int(in3 ? b34 / tlo : 0.0f)));   // (non-negative: ordered as bits)
                 // flush the finished shell segment of partner 1: one atomic per element, density
                 // and target pair (fire-and-forget reductions; a segmented shuffle sum over the
                 // lanes of one shell 3 before them measured slower)
@@ -431,73 +441,77 @@ __global__ void __launch_bounds__(kKThreads) k_exchange(const __grid_constant__ 
                     }
                     any = false;
                 };
-                stage_ent(ring, d12, A.b12, A.cart12, A.t1_12, A.seg12, s12, 0, n12, lane);
+                stage_ent(ring, d12, A.b12, A.cart12, A.t1_12, A.seg12, s12, k1a, n12, lane);
                 cp_async_commit();
                 bool stop = false;
-                for (int kb = 0; kb < n12 && !stop; kb += 32) {
-                    const KEnt<R>* cur = ring + ((kb >> 5) & 1) * 32;
+                int slot = 0;
+                for (int kb = k1a; kb < n12 && !stop; kb += 32, slot ^= 1) {
+                    const KEnt<R>* cur = ring + slot * 32;
                     if (kb + 32 < n12)
-                        stage_ent(ring + (((kb >> 5) + 1) & 1) * 32, d12, A.b12, A.cart12, A.t1_12, A.seg12, s12,
+                        stage_ent(ring + (slot ^ 1) * 32, d12, A.b12, A.cart12, A.t1_12, A.seg12, s12,
                                   kb + 32, n12, lane);
                     cp_async_commit();
                     cp_async_wait<1>();
                     __syncwarp();
                     const int kend = min(32, n12 - kb);
-                    // chg bit l: entry l of the chunk starts a new shell segment (l >= 1)
-                    const int cl = lane < kend ? cur[lane].seg : -1;
-                    const int cl_prev = __shfl_up_sync(0xffffffffu, cl, 1);
-                    const unsigned chg = __ballot_sync(0xffffffffu, lane >= 1 && lane < kend && cl != cl_prev);
-                    for (int j = 0; j < kend; ++j) {
-                        const float b12 = cur[j].b;
+                    // the chunk's entries, one per lane: those that may pass for some lane (b12 times
+                    // the warp's largest b34 / tlo, with room for the roundings; each lane still applies
+                    // its exact screen), and those that start a shell segment
+                    float bl = 0.0f;
+                    int sl = -1;
+                    if (lane < kend) {
+                        bl = cur[lane].b;
+                        sl = cur[lane].seg;
+                    }
+                    int sp = __shfl_up_sync(0xffffffffu, sl, 1);
+                    if (lane == 0) sp = last_seg;
+                    last_seg = __shfl_sync(0xffffffffu, sl, kend - 1);
+                    const bool cand = bl >= thre12 && bl * rmax >= 0.999999f;
+                    unsigned todo = __ballot_sync(0xffffffffu, lane < kend && cand);
+                    // segments are ordered by their largest (first) bound: where one's first entry
+                    // cannot pass, nothing later does
+                    stop = __any_sync(0xffffffffu, lane < kend && sl != sp && !cand);
+                    while (todo) {
+                        const int j = __ffs(todo) - 1;
+                        todo &= todo - 1;
                         const int sg = cur[j].seg;
-                        // can this lane's quartet reach its lower threshold (or any later one of the
-                        // segment / of later segments, whose bounds are not larger)?
-                        const float est = b12 * b34;
-                        const bool can = v3 && est >= tlo;
-                        const bool any_can = b12 >= thre12 && __any_sync(0xffffffffu, can);
                         if (sg != prev_seg) {
                             flush();
                             prev_seg = sg;
                             prev_c1 = cur[j].c;
                             if constexpr (G1 == 2) prev_c1b = cur[j].t1;
-                            // segments are ordered by their largest bound: nothing later passes
-                            if (!any_can) {
-                                stop = true;
-                                break;
+                        }
+                        const float est = cur[j].b * b34;
+                        // (tlo = inf on lanes without a partner 3)
+                        if (est >= tlo && est < thi) {
+                            const KEnt<R> e = cur[j];
+                            nq += dn;   // statistics count density-quartets
+                            any = true;
+                            auto quartet = [&](R(*out)[N1 * N3]) {
+                                k_quartet<L1, L2, L3, L4, R, NG>(A, tab, tmax, tswitch, bscale, asym_t, asym_w, e,
+                                                                 kab34, q, iq, Sx, Sy, Sz, QCx, QCy, QCz, Cx, Cy, Cz,
+                                                                 Dblk, out);
+                            };
+                            if constexpr (G1 == 2) {
+                                // one integral, added to both targets with the entry's weights
+                                R tmp[NG][N1 * N3];
+#pragma unroll
+                                for (int g = 0; g < NG; ++g)
+#pragma unroll
+                                    for (int t = 0; t < N1 * N3; ++t) tmp[g][t] = R(0);
+                                quartet(tmp);
+#pragma unroll
+                                for (int g = 0; g < NG; ++g)
+#pragma unroll
+                                    for (int t = 0; t < N1 * N3; ++t) {
+                                        acc[g][t] = fma(e.w0, tmp[g][t], acc[g][t]);
+                                        accb[g][t] = fma(e.w1, tmp[g][t], accb[g][t]);
+                                    }
+                            } else {
+                                quartet(acc);
                             }
-                        } else if (!any_can) {
-                            // entries of a segment are ordered by bound: skip the rest of this
-                            // segment within the chunk (to the next segment start, or the chunk end)
-                            const unsigned nxt = j == 31 ? 0u : (chg & ~((2u << j) - 1u));
-                            j = (nxt ? __ffs(nxt) - 1 : kend) - 1;
-                            continue;
                         }
-                        const bool pass = can && est < thi;
-                        if (!__any_sync(0xffffffffu, pass)) continue;
-                        if (!pass) continue;
-                        const KEnt<R> e = cur[j];
-                        nq += dn;   // statistics count density-quartets
-                        any = true;
-                        if constexpr (G1 == 2) {
-                            // one integral, added to both targets with the entry's weights
-                            R tmp[NG][N1 * N3];
-#pragma unroll
-                            for (int g = 0; g < NG; ++g)
-#pragma unroll
-                                for (int t = 0; t < N1 * N3; ++t) tmp[g][t] = R(0);
-                            k_quartet<L1, L2, L3, L4, R, NG>(A, tab, tmax, asym_t, asym_w, e, kab34, q, iq, Sx, Sy,
-                                                             Sz, QCx, QCy, QCz, Cx, Cy, Cz, Dblk, tmp);
-#pragma unroll
-                            for (int g = 0; g < NG; ++g)
-#pragma unroll
-                                for (int t = 0; t < N1 * N3; ++t) {
-                                    acc[g][t] = fma(e.w0, tmp[g][t], acc[g][t]);
-                                    accb[g][t] = fma(e.w1, tmp[g][t], accb[g][t]);
-                                }
-                        } else {
-                            k_quartet<L1, L2, L3, L4, R, NG>(A, tab, tmax, asym_t, asym_w, e, kab34, q, iq, Sx, Sy,
-                                                             Sz, QCx, QCy, QCz, Cx, Cy, Cz, Dblk, acc);
-                        }
+                        __syncwarp();   // the lanes that computed rejoin the others
                     }
                     __syncwarp();   // the next chunk's prefetch refills this slot
                 }
@@ -566,8 +580,9 @@ void launch_k(Context* ctx, const KArgs& A, long cap, bool fp32)
     if (cap == 0 || A.ng < 1) return;
     const int per_group = std::min(A.ng, kKBatch);
     int per_sm = ctx->tune.k_ctas_per_sm[fp32 ? 1 : 0][L1][L2][L3][L4];
+    // (a class of few tasks runs up to A.split partner-1 stripes of each)
     auto grid_for = [&](int nsub) {
-        const long want = (cap * nsub + kKWarps - 1) / kKWarps;
+        const long want = (cap * nsub * A.split + kKWarps - 1) / kKWarps;
         return (unsigned) std::min<long>(want, (long) ctx->nsm * (per_sm > 0 ? per_sm : 16));
     };
     KArgs B = A;

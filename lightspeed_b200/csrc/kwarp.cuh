@@ -94,6 +94,7 @@ __global__ void __launch_bounds__(kKThreads, 4) k_exchange_warp(const __grid_con
     const double* tab = static_cast<const double*>(A.rys);
     const double* asym_t = static_cast<const double*>(A.asym_t);
     const double* asym_w = static_cast<const double*>(A.asym_w);
+    const double bscale = A.nbin / A.tmax;
     const float thre12 = A.sc->thre12, thre34 = A.sc->thre34;
     const double thr_lo = (double) A.thr_lo, thr_hi = (double) A.thr_hi;
     // offsets of shell 2's components in the tables of the three directions
@@ -228,7 +229,7 @@ __global__ void __launch_bounds__(kKThreads, 4) k_exchange_warp(const __grid_con
                         if (lane < 3 * Sh::RG && r0 + rl < NR) {
                             // 2-D integrals I(a, c) of root r0 + rl in direction dl
                             double t2, w;
-                            rys_root(T, tab, NR, r0 + rl, A.nbin, A.tmax, asym_t, asym_w, t2, w);
+                            rys_root(T, tab, NR, r0 + rl, A.nbin, A.tmax, bscale, asym_t, asym_w, t2, w);
                             const double u = t2 * d2 * ipq, qu = q * u, pu = p * u;
                             const double b00 = 0.5 * u, b10 = 0.5 * ip * (1.0 - qu), b01 = 0.5 * iq * (1.0 - pu);
                             const double PQd = dl == 0 ? PQ[0] : (dl == 1 ? PQ[1] : PQ[2]);

@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(kXThreads) k_xgrad(const __grid_constant__ XGr
     int* pend = queue_all[threadIdx.x >> 5];
     const float thre = A.sc->thre12;
     const double dmax = __longlong_as_double((long long) A.sc->dmax_bits);
-    const double thr = (double) A.thr;
+    const double thr = (double) A.thr, bscale = A.nbin / A.tmax;
     for (;;) {
         unsigned unit = 0;
         if (lane == 0) unit = atomicAdd(A.queue, 1u);
@@ -191,7 +191,7 @@ __global__ void __launch_bounds__(kXThreads) k_xgrad(const __grid_constant__ XGr
                     f *= sqrt(d2);
                 }
                 double t2[NR], w[NR];
-                rys_eval<NR, double>(rho * d2 * RR, tab, A.nbin, A.tmax, A.asym_t, A.asym_w, t2, w);
+                rys_eval<NR, double>(rho * d2 * RR, tab, A.nbin, A.tmax, bscale, A.asym_t, A.asym_w, t2, w);
                 // one root after another: slot 0 is the root in use and the rest shift down,
                 // so the arrays keep static indices and the code one copy of the root
 #pragma unroll 1
@@ -280,7 +280,7 @@ __global__ void __launch_bounds__(kXThreads) k_xgrad_warp(const __grid_constant_
     const int lane = threadIdx.x & 31;
     const float thre = A.sc->thre12;
     const double dmax = __longlong_as_double((long long) A.sc->dmax_bits);
-    const double thr = (double) A.thr;
+    const double thr = (double) A.thr, bscale = A.nbin / A.tmax;
     const int rl = lane < 3 * NR ? lane / 3 : 0, dl = lane % 3;   // this lane's root and direction
     for (;;) {
         unsigned unit = 0;
@@ -338,7 +338,7 @@ __global__ void __launch_bounds__(kXThreads) k_xgrad_warp(const __grid_constant_
                     __syncwarp();
                     if (lane < 3 * NR) {
                         double t2, w;
-                        rys_root(rho * d2 * RR, A.rys, NR, rl, A.nbin, A.tmax, A.asym_t, A.asym_w, t2, w);
+                        rys_root(rho * d2 * RR, A.rys, NR, rl, A.nbin, A.tmax, bscale, A.asym_t, A.asym_w, t2, w);
                         const double u = t2 * d2 * ipq, qu = q * u, pu = p * u;
                         const double b00 = 0.5 * u, b10 = 0.5 * B.ip * (1.0 - qu), b01 = 0.5 * iq * (1.0 - pu);
                         const double c00 = PAd - qu * PQd, d00 = QCd + pu * PQd;

@@ -128,11 +128,6 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
-// Half-range Gauss-Hermite nodes and weights of the asymptotic Rys rules,
-// [nrys][root], in constant memory (read with uniform indices).
-static __constant__ double c_rys_asym_t[(LSJK_RYS_NMAX + 1) * LSJK_RYS_NMAX] = {LSJK_RYS_ASYM_T_LIST};
-static __constant__ double c_rys_asym_w[(LSJK_RYS_NMAX + 1) * LSJK_RYS_NMAX] = {LSJK_RYS_ASYM_W_LIST};
-
 // 1/sqrt(T) in FP64 for T > 0: the FP32 estimate refined by two Newton steps
 // r <- r (3 - T r^2) / 2 (relative error ~1e-16; the FP32 paths' switch
 // region never sees T near 0 or beyond the float range).
@@ -186,15 +181,16 @@ __device__ __forceinline__ void boys_eval(R T, const R* __restrict__ tab, R* __r
 
 // Rys roots (returned as t^2) and weights of the N-point rule at T. `tab` is the
 // per-rule block [2N][nbin][8] (roots t, then ln w; for N = 1 the weight
-// w = F_0(T) itself, so the one-root classes need no exponential);
+// w = F_0(T) itself, so the one-root classes need no exponential); `bscale` is
+// nbin / tmax, formed once per thread and not divided out for every quartet;
 // `asym_t/asym_w` hold the half-range Gauss-Hermite limit used for T >= tmax.
 template <int N, typename R>
-__device__ __forceinline__ void rys_eval(R T, const R* __restrict__ tab, int nbin, R tmax,
+__device__ __forceinline__ void rys_eval(R T, const R* __restrict__ tab, int nbin, R tmax, R bscale,
                                          const R* __restrict__ asym_t, const R* __restrict__ asym_w,
                                          R* __restrict__ t2, R* __restrict__ w)
 {
     if (T < tmax) {
-        const R u = T * (R(nbin) / tmax);
+        const R u = T * bscale;
         int b = static_cast<int>(u);
         b = b < nbin - 1 ? b : nbin - 1;
         const R x = R(2) * (u - R(b)) - R(1);
@@ -216,14 +212,60 @@ __device__ __forceinline__ void rys_eval(R T, const R* __restrict__ tab, int nbi
     }
 }
 
+// The asymptotic Rys nodes as pairs of floats: squares of the roots (hi + lo) and weights.
+struct RysAsymPairs {
+    static constexpr int n = (LSJK_RYS_NMAX + 1) * LSJK_RYS_NMAX;
+    float sh[n], sl[n], wh[n], wl[n];
+};
+__host__ __device__ constexpr RysAsymPairs make_rys_asym_pairs()
+{
+    constexpr double t[RysAsymPairs::n] = {LSJK_RYS_ASYM_T_LIST};
+    constexpr double w[RysAsymPairs::n] = {LSJK_RYS_ASYM_W_LIST};
+    RysAsymPairs P{};
+    for (int i = 0; i < RysAsymPairs::n; ++i) {
+        P.sh[i] = (float) (t[i] * t[i]);
+        P.sl[i] = (float) (t[i] * t[i] - (double) P.sh[i]);
+        P.wh[i] = (float) w[i];
+        P.wl[i] = (float) (w[i] - (double) P.wh[i]);
+    }
+    return P;
+}
+static __constant__ RysAsymPairs c_rys_asym_pairs = make_rys_asym_pairs();
+
+// Roots t^2 = s^2 / T and weights w = h / sqrt(T) of the asymptotic N-point rule at
+// T = rho d2 RR, rounded to FP32 once: T, 1/T and 1/sqrt(T) are carried as unevaluated
+// sums of two floats (products split exactly by fma; one Newton step on the hardware
+// rsqrt, whose residual e = 1 - T r^2 ~ 2^-22 is itself exact to ~2^-47). The results
+// equal the FP64 evaluation rounded to FP32 to within 2^-24 (1 + 1e-5) relative. In FP64
+// this took eight conversions and a dozen FP64 operations per quartet: half the
+// conversion pipe's load of the light classes.
+template <int N>
+__device__ __forceinline__ void rys_asym_pairs(float rho, float d2, float RR, float* __restrict__ t2,
+                                               float* __restrict__ w)
+{
+    const float a = rho * d2, al = fmaf(rho, d2, -a);
+    const float Th = a * RR, Tl = fmaf(al, RR, fmaf(a, RR, -Th));
+    const float r = rsqrtf(Th);
+    const float s = r * r, sl = fmaf(r, r, -s);
+    const float e = fmaf(-Th, sl, fmaf(-Tl, s, fmaf(-Th, s, 1.0f)));
+    const float sc = fmaf(s, e, sl);     // 1/T = s + sc
+    const float rc = 0.5f * r * e;       // 1/sqrt(T) = r + rc
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        const int k = N * LSJK_RYS_NMAX + i;
+        t2[i] = fmaf(c_rys_asym_pairs.sh[k], s, fmaf(c_rys_asym_pairs.sh[k], sc, c_rys_asym_pairs.sl[k] * s));
+        w[i] = fmaf(c_rys_asym_pairs.wh[k], r, fmaf(c_rys_asym_pairs.wh[k], rc, c_rys_asym_pairs.wl[k] * r));
+    }
+}
+
 // Root i alone of the N-point rule (FP64), for lanes that share a quartet's roots out.
 __device__ __forceinline__ void rys_root(double T, const double* __restrict__ tab, int N, int i, int nbin, double tmax,
-                                         const double* __restrict__ asym_t, const double* __restrict__ asym_w,
+                                         double bscale, const double* __restrict__ asym_t, const double* __restrict__ asym_w,
                                          double& t2, double& w)
 {
     double t;
     if (T < tmax) {
-        const double u = T * (nbin / tmax);
+        const double u = T * bscale;
         int b = static_cast<int>(u);
         b = b < nbin - 1 ? b : nbin - 1;
         const double x = 2.0 * (u - b) - 1.0;
