@@ -16,6 +16,7 @@
 #include <atomic>
 #include <cstdint>
 #include <cstdio>
+#include <functional>
 #include <string>
 #include <vector>
 #include <memory>
@@ -60,11 +61,18 @@ template <typename T>
 struct DBuf {
     T* p = nullptr;
     size_t n = 0;
+    bool own = true;      // false: a slice of another buffer (see slice)
     DBuf() = default;
     DBuf(const DBuf&) = delete;
     DBuf& operator=(const DBuf&) = delete;
-    DBuf(DBuf&& o) noexcept : p(o.p), n(o.n) { o.p = nullptr; o.n = 0; }
-    DBuf& operator=(DBuf&& o) noexcept { release(); p = o.p; n = o.n; o.p = nullptr; o.n = 0; return *this; }
+    DBuf(DBuf&& o) noexcept : p(o.p), n(o.n), own(o.own) { o.p = nullptr; o.n = 0; }
+    DBuf& operator=(DBuf&& o) noexcept
+    {
+        release();
+        p = o.p; n = o.n; own = o.own;
+        o.p = nullptr; o.n = 0;
+        return *this;
+    }
     ~DBuf() { release(); }
     void alloc(size_t count) {
         release();
@@ -81,7 +89,30 @@ struct DBuf {
         alloc(h.size());
         if (!h.empty()) LSJK_CUDA(cudaMemcpyAsync(p, h.data(), sizeof(T) * h.size(), cudaMemcpyHostToDevice, s));
     }
-    void release() { if (p) cudaFree(p); p = nullptr; n = 0; }
+    // `count` elements at `at`, inside a buffer that outlives this one
+    void slice(T* at, size_t count) { release(); p = count ? at : nullptr; n = count; own = false; }
+    void release() { if (p && own) cudaFree(p); p = nullptr; n = 0; own = true; }
+};
+
+// The arrays of one object as slices of one allocation: add() each array, then
+// allocate() once. A cudaMalloc and a cudaFree per array (31 for a pair list, 88 for its
+// K-invert rows) took most of a pair list's set-up time.
+struct Arena {
+    DBuf<char>& buf;
+    size_t bytes = 0;
+    std::vector<std::pair<size_t, std::function<void(char*)>>> parts;
+    explicit Arena(DBuf<char>& b) : buf(b) {}
+    template <typename T>
+    void add(DBuf<T>& d, size_t count)
+    {
+        parts.emplace_back(bytes, [&d, count](char* at) { d.slice(reinterpret_cast<T*>(at), count); });
+        bytes += (sizeof(T) * count + 255) & ~size_t(255);
+    }
+    void allocate()
+    {
+        buf.alloc(bytes);
+        for (auto& q : parts) q.second(buf.p + q.first);
+    }
 };
 
 struct Context;
@@ -151,7 +182,6 @@ struct JBraClass {
 // K-invert rows of one (L_indexed, L_partner) class: for every primitive of
 // the indexed basis, the [start, start+len) slice of the partner arrays.
 struct KInvClass {
-    int nent = 0;
     DBuf<int> row_start, row_len;    // per indexed primitive (len 0: no partners)
 };
 
@@ -175,11 +205,11 @@ struct KInvData {
     DBuf<float> pw0_32, pw1_32;
     DBuf<double> pe;                   // partner's exponent (the K gradient's derivatives)
     DBuf<int> patom;                   // partner's atom
-    DBuf<int> pidx;                    // partner's primitive index
 };
 
 struct PairList {
     Context* ctx = nullptr;
+    DBuf<char> arena, kinv_arena;      // what the arrays below are slices of
     const Basis* b1 = nullptr;
     const Basis* b2 = nullptr;
     bool symm = false;
@@ -192,10 +222,11 @@ struct PairList {
     std::vector<long> cls_off;         // offsets into the sorted arrays (size nclass+1)
     std::vector<float> cls_max;        // first (largest) bound of each class
     double max_bound = 0.0;            // PairListUtil::max_bound
-    // J bra view per Hermite class
-    JBraClass jb[kNHerm];
+    // J bra view per Hermite class (slices of the arrays over all classes)
+    JBraClass jall, jb[kNHerm];
     // K-invert rows: [L_indexed][L_partner]
     KInvClass kinv[kNL][kNL];
+    DBuf<int> row_start, row_len;      // every class's rows, one after another
     KInvData kdat;     // rows grouped by contracted shell (segments): the partner-1 side of K
     KInvData kdat_b;   // the same rows, entries by bound only: the partner-3 side of K
     bool kinv_built = false;

@@ -203,12 +203,11 @@ std::shared_ptr<PairList> PairList::build_schwarz(const std::shared_ptr<Basis>& 
     long k = 0;
     while (k < n) {
         long e = k;
+        while (e < n && L1[e] == L1[k] && L2[e] == L2[k]) ++e;
         std::vector<Pair> pairs;
-        while (e < n && L1[e] == L1[k] && L2[e] == L2[k]) {
-            pairs.emplace_back(&P1[p1[e]], &P2[p2[e]], b[e]);
-            ++e;
-        }
-        pl->pairlists_.emplace_back(is_symmetric, L1[k], L2[k], pairs);
+        pairs.reserve(e - k);
+        for (long q = k; q < e; ++q) pairs.emplace_back(&P1[p1[q]], &P2[p2[q]], b[q]);
+        pl->pairlists_.emplace_back(is_symmetric, L1[k], L2[k], std::move(pairs));
         k = e;
     }
     return pl;

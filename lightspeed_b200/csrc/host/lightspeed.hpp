@@ -116,8 +116,8 @@ private:
 
 class PairListL {
 public:
-    PairListL(bool is_symmetric, int L1, int L2, const std::vector<Pair>& pairs)
-        : symm_(is_symmetric), L1_(L1), L2_(L2), pairs_(pairs) {}
+    PairListL(bool is_symmetric, int L1, int L2, std::vector<Pair> pairs)
+        : symm_(is_symmetric), L1_(L1), L2_(L2), pairs_(std::move(pairs)) {}
     bool is_symmetric() const { return symm_; }
     int L1() const { return L1_; }
     int L2() const { return L2_; }

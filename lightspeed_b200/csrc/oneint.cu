@@ -12,6 +12,8 @@
 // adds it with FP64 atomics into the Cartesian matrix (both triangles for a
 // symmetric list, 1/2 on a primitive's pair with itself, as the reference's
 // symmetric pair-list consumers). The pure transform follows on the device.
+#include <algorithm>
+#include <optional>
 #include "engine.cuh"
 #include "hermite.cuh"
 #include "quartet_loops.cuh"   // herm_pos
@@ -136,7 +138,8 @@ __global__ void __launch_bounds__(128) k_oneint(const __grid_constant__ OneArgs 
         for (int k = 0; k < H; ++k) Rs[k] = 0.0;
         double R[H];
         double F[L + 1];
-        for (int C = 0; C < A.natom; ++C) {
+        // the charges are shared out over grid.y (each slice adds its part of the block)
+        for (int C = blockIdx.y; C < A.natom; C += gridDim.y) {
             const double Zc = A.xyzc[4 * C + 3];
             if (Zc == 0.0) continue;
             const double X = P[0] - A.xyzc[4 * C], Y = P[1] - A.xyzc[4 * C + 1], Z = P[2] - A.xyzc[4 * C + 2];
@@ -184,7 +187,13 @@ __global__ void __launch_bounds__(128) k_oneint(const __grid_constant__ OneArgs 
 template <int KIND>
 void launch_one(Context* ctx, const OneArgs& A, int LA, int LB)
 {
-    const unsigned grid = (unsigned) ((A.n + 127) / 128);
+    // V: a thread walks the charges one after another, so they are split until there are two
+    // CTAs per multiprocessor (a d|d class of a few hundred pairs fills two CTAs: 308 us of
+    // the 790 us of V kernels for C20H42/cc-pVDZ unsplit)
+    const unsigned tiles = (unsigned) ((A.n + 127) / 128);
+    unsigned slices = 1;
+    if (KIND == kOneV) slices = std::min<unsigned>(std::max(1, A.natom), (2u * ctx->nsm + tiles - 1) / tiles);
+    const dim3 grid(tiles, slices);
     cudaStream_t s = ctx->stream;
 #define LSJK_ONE(a, b)                                                     \
     if (LA == a && LB == b) {                                              \
@@ -205,6 +214,9 @@ void one_electron(Context* ctx, int kind, const PairList* pl, const Ewald* ew, c
                   double* Xcart)
 {
     if (ew && ew->alpha.size() > 4) throw Error(LSJK_EINVAL, "IntBox::potential: at most 4 Ewald terms");
+    // the classes of V overlap on the auxiliary streams; those of S and T are too short to
+    const bool par = kind == kOneV;
+    if (par) fork_aux(ctx, pl->npair);
     for (size_t c = 0; c + 1 < pl->cls_off.size(); ++c) {
         OneArgs A{};
         A.p1 = pl->p1.p;
@@ -218,6 +230,8 @@ void one_electron(Context* ctx, int kind, const PairList* pl, const Ewald* ew, c
         A.X = Xcart;
         A.ld = pl->b2->ncart;
         const int LA = pl->cls_L1[c], LB = pl->cls_L2[c];
+        std::optional<OnAux> on;
+        if (par) on.emplace(ctx, (int) c);
         if (kind == kOneV) {
             A.xyzc = xyzc;
             A.natom = natom;
@@ -234,6 +248,7 @@ void one_electron(Context* ctx, int kind, const PairList* pl, const Ewald* ew, c
             launch_one<kOneS>(ctx, A, LA, LB);
         }
     }
+    if (par) join_aux(ctx);
 }
 
 } // namespace lsjk

@@ -106,6 +106,22 @@ __global__ void k_gather_pairs(const PairTmp* __restrict__ in, const int* __rest
     b[k] = t.b;
 }
 
+// For the classes c < ncls of keys sorted ascending by (class << 32 | ~bound bits): the
+// first entry of class c (start[c], up to start[ncls] = n) and its key's low half.
+__global__ void k_class_starts(const unsigned long long* __restrict__ key, int n, int ncls, int* __restrict__ start,
+                               unsigned* __restrict__ low)
+{
+    const int c = threadIdx.x;
+    if (c > ncls) return;
+    int lo = 0, hi = n;
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if ((key[mid] >> 32) < (unsigned long long) c) lo = mid + 1; else hi = mid;
+    }
+    start[c] = c == ncls ? n : lo;
+    low[c] = lo < n ? (unsigned) key[lo] : 0u;
+}
+
 // Gaussian product geometry of a pair: p = e1 + e2, P = (e1 A + e2 B) / p.
 __global__ void k_pair_geom(BasisView b1, BasisView b2, const int* __restrict__ p1,
                             const int* __restrict__ p2, int n, double* __restrict__ geom)
@@ -221,8 +237,7 @@ __global__ void k_kinv_fill(const KEnt* __restrict__ e, const int* __restrict__ 
                             int* __restrict__ pcart, float* __restrict__ pb, int* __restrict__ pt1,
                             int* __restrict__ pseg, double* __restrict__ pw0, double* __restrict__ pw1,
                             float* __restrict__ pw0_32, float* __restrict__ pw1_32, double* __restrict__ pe,
-                            int* __restrict__ patom, int* __restrict__ pidx, int* __restrict__ rstart,
-                            int* __restrict__ rlen, int nrow)
+                            int* __restrict__ patom, int* __restrict__ rstart, int* __restrict__ rlen, int nrow)
 {
     long k = blockIdx.x * (long) blockDim.x + threadIdx.x;
     if (k >= n) return;
@@ -248,7 +263,6 @@ __global__ void k_kinv_fill(const KEnt* __restrict__ e, const int* __restrict__ 
     pw1_32[k] = (float) bpart.w1[j];
     pe[k] = ej;
     patom[k] = bpart.atom[j];
-    pidx[k] = j;
     pb[k] = t.b;
     long r = (long) t.cls * nrow + i;
     bool first = (k == 0);
@@ -287,9 +301,17 @@ void build_pairlist(Context* ctx, PairList* pl)
     LSJK_CUDA(cudaStreamSynchronize(s));
     long n = (long) hn;
     pl->npair = n;
-    pl->p1.alloc(n);
-    pl->p2.alloc(n);
-    pl->bound.alloc(n);
+    {
+        Arena A(pl->arena);
+        A.add(pl->p1, n);
+        A.add(pl->p2, n);
+        A.add(pl->bound, n);
+        A.add(pl->jall.p1, n);
+        A.add(pl->jall.p2, n);
+        A.add(pl->jall.bound, n);
+        A.add(pl->jall.geom, 4 * n);
+        A.allocate();
+    }
     pl->cls_L1.clear();
     pl->cls_L2.clear();
     pl->cls_off.assign(1, 0);
@@ -315,57 +337,55 @@ void build_pairlist(Context* ctx, PairList* pl)
     LSJK_CUDA(cudaGetLastError());
 
     // class offsets and the leading (largest) bound of each class
-    std::vector<unsigned long long> hk(n);
-    LSJK_CUDA(cudaMemcpyAsync(hk.data(), k2s, sizeof(unsigned long long) * n, cudaMemcpyDeviceToHost, s));
-    LSJK_CUDA(cudaStreamSynchronize(s));
-    for (long k = 0; k < n; ++k) {
-        unsigned cls = (unsigned) (hk[k] >> 32);
-        if (k == 0 || cls != (unsigned) (hk[k - 1] >> 32)) {
-            if (k > 0) pl->cls_off.push_back(k);
-            pl->cls_L1.push_back((int) cls / nL2);
-            pl->cls_L2.push_back((int) cls % nL2);
-            unsigned bits = ~(unsigned) (hk[k] & 0xffffffffu);
-            float b;
-            memcpy(&b, &bits, sizeof(b));
-            pl->cls_max.push_back(b);
-            pl->max_bound = std::max(pl->max_bound, (double) b);
-        }
-    }
-    pl->cls_off.push_back(n);
+    constexpr int kMaxCls = 128;   // (s to n shells on either side)
+    const int ncls = (b1->maxL + 1) * nL2, nherm = b1->maxL + b2->maxL + 1;
+    if (ncls >= kMaxCls || nherm >= kMaxCls)
+        throw Error(LSJK_ENOTSUPP, "PairList: angular momentum above d is not supported by the GPU J/K kernels");
+    int* starts = take<int>(ctx, 4 * kMaxCls);
+    unsigned* lows = reinterpret_cast<unsigned*>(starts + 2 * kMaxCls);
+    k_class_starts<<<1, kMaxCls, 0, s>>>(k2s, (int) n, ncls, starts, lows);
 
     // J bra view: stable re-sort of pass-1 order by (L1+L2, bound desc)
     int* perm_h = take<int>(ctx, n);
     k_keys_herm<<<nblk(n, 256), 256, 0, s>>>(tmp, perm1, n, b1->dL.p, b2->dL.p, k2);
     radix_sort_pairs(ctx, k2, k2s, perm1, perm_h, n, 40);
-    std::vector<unsigned long long> hh(n);
-    LSJK_CUDA(cudaMemcpyAsync(hh.data(), k2s, sizeof(unsigned long long) * n, cudaMemcpyDeviceToHost, s));
-    LSJK_CUDA(cudaStreamSynchronize(s));
-    long start = 0;
-    for (int h = 0; h < kNHerm + 4; ++h) {
-        long end = start;
-        while (end < n && (int) (hh[end] >> 32) == h) ++end;
-        long cnth = end - start;
-        if (h < kNHerm) {
-            JBraClass& jb = pl->jb[h];
-            jb.n = (int) cnth;
-            jb.p1.alloc(cnth);
-            jb.p2.alloc(cnth);
-            jb.bound.alloc(cnth);
-            jb.geom.alloc(4 * cnth);
-            if (cnth) {
-                k_gather_pairs<<<nblk(cnth, 256), 256, 0, s>>>(tmp, perm_h + start, cnth, jb.p1.p, jb.p2.p,
-                                                               jb.bound.p);
-                k_pair_geom<<<nblk(cnth, 256), 256, 0, s>>>(b1->view(), b2->view(), jb.p1.p, jb.p2.p,
-                                                            (int) cnth, jb.geom.p);
-            }
-        } else if (cnth) {
-            throw Error(LSJK_ENOTSUPP, "PairList: angular momentum above d is not supported by the GPU J/K kernels");
-        }
-        start = end;
-    }
+    k_class_starts<<<1, kMaxCls, 0, s>>>(k2s, (int) n, nherm, starts + kMaxCls, lows + kMaxCls);
+    k_gather_pairs<<<nblk(n, 256), 256, 0, s>>>(tmp, perm_h, n, pl->jall.p1.p, pl->jall.p2.p, pl->jall.bound.p);
+    k_pair_geom<<<nblk(n, 256), 256, 0, s>>>(b1->view(), b2->view(), pl->jall.p1.p, pl->jall.p2.p, (int) n,
+                                            pl->jall.geom.p);
     LSJK_CUDA(cudaGetLastError());
+    int hst[4 * kMaxCls];
+    LSJK_CUDA(cudaMemcpyAsync(hst, starts, sizeof(hst), cudaMemcpyDeviceToHost, s));
     LSJK_CUDA(cudaStreamSynchronize(s));
-    ctx->stats.kernel_launches += 8;
+    for (int c = 0; c < ncls; ++c) {
+        if (hst[c + 1] == hst[c]) continue;
+        if (hst[c] > 0) pl->cls_off.push_back(hst[c]);
+        pl->cls_L1.push_back(c / nL2);
+        pl->cls_L2.push_back(c % nL2);
+        const unsigned bits = ~(unsigned) hst[2 * kMaxCls + c];
+        float b;
+        memcpy(&b, &bits, sizeof(b));
+        pl->cls_max.push_back(b);
+        pl->max_bound = std::max(pl->max_bound, (double) b);
+    }
+    pl->cls_off.push_back(n);
+    const int* hh = hst + kMaxCls;
+    for (int h = 0; h < nherm; ++h) {
+        const int st = hh[h], cnt = hh[h + 1] - st;
+        if (h >= kNHerm) {
+            if (cnt && h < kNHerm + 4)
+                throw Error(LSJK_ENOTSUPP,
+                            "PairList: angular momentum above d is not supported by the GPU J/K kernels");
+            continue;
+        }
+        JBraClass& jb = pl->jb[h];
+        jb.n = cnt;
+        jb.p1.slice(pl->jall.p1.p + st, cnt);
+        jb.p2.slice(pl->jall.p2.p + st, cnt);
+        jb.bound.slice(pl->jall.bound.p + st, cnt);
+        jb.geom.slice(pl->jall.geom.p + 4L * st, 4 * (size_t) cnt);
+    }
+    ctx->stats.kernel_launches += 10;
 }
 
 void build_kinv(Context* ctx, PairList* pl)
@@ -379,13 +399,25 @@ void build_kinv(Context* ctx, PairList* pl)
     long cap = pl->symm ? 2 * n : n;
     int nrow = bidx->nprim;
     KInvData& kd = pl->kdat;
-    for (int a = 0; a < kNL; ++a)
-        for (int b = 0; b < kNL; ++b) {
-            pl->kinv[a][b].row_start.alloc(nrow);
-            pl->kinv[a][b].row_len.alloc(nrow);
-            pl->kinv[a][b].nent = 0;
-        }
-    if (n == 0) { kd.nent = 0; pl->kinv_built = true; return; }
+    const size_t nrows = (size_t) kNL * kNL * nrow;
+    auto rows = [&] {
+        for (int a = 0; a < kNL; ++a)
+            for (int b = 0; b < kNL; ++b) {
+                const long off = (long) (a * kNL + b) * nrow;
+                pl->kinv[a][b].row_start.slice(pl->row_start.p + off, nrow);
+                pl->kinv[a][b].row_len.slice(pl->row_len.p + off, nrow);
+            }
+    };
+    if (n == 0) {
+        Arena A(pl->kinv_arena);
+        A.add(pl->row_start, nrows);
+        A.add(pl->row_len, nrows);
+        A.allocate();
+        rows();
+        kd.nent = 0;
+        pl->kinv_built = true;
+        return;
+    }
     KEnt* ent = take<KEnt>(ctx, cap);
     unsigned long long* cnt = take<unsigned long long>(ctx, 1);
     LSJK_CUDA(cudaMemsetAsync(cnt, 0, sizeof(unsigned long long), s));
@@ -396,13 +428,26 @@ void build_kinv(Context* ctx, PairList* pl)
     LSJK_CUDA(cudaStreamSynchronize(s));
     long m = (long) hn;
     kd.nent = m;
-    kd.kab.alloc(m); kd.p.alloc(m); kd.ip.alloc(m); kd.px.alloc(m); kd.py.alloc(m); kd.pz.alloc(m);
-    kd.ax.alloc(m); kd.ay.alloc(m); kd.az.alloc(m);
-    kd.kab32.alloc(m); kd.p32.alloc(m); kd.ip32.alloc(m); kd.px32.alloc(m); kd.py32.alloc(m);
-    kd.pz32.alloc(m); kd.ax32.alloc(m); kd.ay32.alloc(m); kd.az32.alloc(m);
-    kd.pcart.alloc(m); kd.pbound.alloc(m);
-    kd.pt1.alloc(m); kd.pseg.alloc(m); kd.pw0.alloc(m); kd.pw1.alloc(m); kd.pw0_32.alloc(m); kd.pw1_32.alloc(m);
-    kd.pe.alloc(m); kd.patom.alloc(m); kd.pidx.alloc(m);
+    // the rows grouped by contracted shell, and the bound-ordered copy (same rows, so the
+    // same row tables)
+    KInvData& kb_ = pl->kdat_b;
+    kb_.nent = m;
+    {
+        Arena A(pl->kinv_arena);
+        A.add(pl->row_start, nrows);
+        A.add(pl->row_len, nrows);
+        for (KInvData* d : {&kd, &kb_}) {
+            for (DBuf<double>* x : {&d->kab, &d->p, &d->ip, &d->px, &d->py, &d->pz, &d->ax, &d->ay, &d->az, &d->pw0,
+                                    &d->pw1, &d->pe})
+                A.add(*x, m);
+            for (DBuf<float>* x : {&d->kab32, &d->p32, &d->ip32, &d->px32, &d->py32, &d->pz32, &d->ax32, &d->ay32,
+                                   &d->az32, &d->pw0_32, &d->pw1_32, &d->pbound})
+                A.add(*x, m);
+            for (DBuf<int>* x : {&d->pcart, &d->pt1, &d->pseg, &d->patom}) A.add(*x, m);
+        }
+        A.allocate();
+    }
+    rows();
     unsigned long long* ka = take<unsigned long long>(ctx, m);
     unsigned long long* kas = take<unsigned long long>(ctx, m);
     int* va = take<int>(ctx, m);
@@ -424,28 +469,17 @@ void build_kinv(Context* ctx, PairList* pl)
     int* perm = take<int>(ctx, m);
     k_kinv_key3<<<nblk(m, 256), 256, 0, s>>>(ent, pb2, kbs, m, kc);
     radix_sort_pairs(ctx, kc, kcs, pb2, perm, m, 52);
-    // row tables live in one [class][row] block per class
-    int* rstart = take<int>(ctx, (long) kNL * kNL * nrow);
-    int* rlen = take<int>(ctx, (long) kNL * kNL * nrow);
-    LSJK_CUDA(cudaMemsetAsync(rstart, 0, sizeof(int) * kNL * kNL * nrow, s));
-    LSJK_CUDA(cudaMemsetAsync(rlen, 0, sizeof(int) * kNL * kNL * nrow, s));
+    // row tables: one [class][row] block
+    int *rstart = pl->row_start.p, *rlen = pl->row_len.p;
+    LSJK_CUDA(cudaMemsetAsync(rstart, 0, sizeof(int) * nrows, s));
+    LSJK_CUDA(cudaMemsetAsync(rlen, 0, sizeof(int) * nrows, s));
     k_kinv_fill<<<nblk(m, 256), 256, 0, s>>>(ent, perm, m, bidx->view(), bpart->view(), nullptr, kd.kab.p, kd.p.p,
                                             kd.ip.p, kd.px.p, kd.py.p, kd.pz.p, kd.ax.p, kd.ay.p, kd.az.p,
                                             kd.kab32.p, kd.p32.p, kd.ip32.p, kd.px32.p, kd.py32.p, kd.pz32.p,
                                             kd.ax32.p, kd.ay32.p, kd.az32.p, kd.pcart.p, kd.pbound.p, kd.pt1.p,
                                             kd.pseg.p, kd.pw0.p, kd.pw1.p, kd.pw0_32.p, kd.pw1_32.p, kd.pe.p,
-                                            kd.patom.p, kd.pidx.p, rstart, rlen, nrow);
+                                            kd.patom.p, rstart, rlen, nrow);
     LSJK_CUDA(cudaGetLastError());
-    // the bound-ordered copy (same rows, so the same row tables)
-    KInvData& kb_ = pl->kdat_b;
-    kb_.nent = m;
-    kb_.kab.alloc(m); kb_.p.alloc(m); kb_.ip.alloc(m); kb_.px.alloc(m); kb_.py.alloc(m); kb_.pz.alloc(m);
-    kb_.ax.alloc(m); kb_.ay.alloc(m); kb_.az.alloc(m);
-    kb_.kab32.alloc(m); kb_.p32.alloc(m); kb_.ip32.alloc(m); kb_.px32.alloc(m); kb_.py32.alloc(m);
-    kb_.pz32.alloc(m); kb_.ax32.alloc(m); kb_.ay32.alloc(m); kb_.az32.alloc(m);
-    kb_.pcart.alloc(m); kb_.pbound.alloc(m);
-    kb_.pt1.alloc(m); kb_.pseg.alloc(m); kb_.pw0.alloc(m); kb_.pw1.alloc(m); kb_.pw0_32.alloc(m);
-    kb_.pw1_32.alloc(m); kb_.pe.alloc(m); kb_.patom.alloc(m); kb_.pidx.alloc(m);
     int* rstart_b = take<int>(ctx, (long) kNL * kNL * nrow);
     int* rlen_b = take<int>(ctx, (long) kNL * kNL * nrow);
     LSJK_CUDA(cudaMemsetAsync(rstart_b, 0, sizeof(int) * kNL * kNL * nrow, s));
@@ -455,16 +489,8 @@ void build_kinv(Context* ctx, PairList* pl)
                                             kb_.az.p, kb_.kab32.p, kb_.p32.p, kb_.ip32.p, kb_.px32.p, kb_.py32.p,
                                             kb_.pz32.p, kb_.ax32.p, kb_.ay32.p, kb_.az32.p, kb_.pcart.p,
                                             kb_.pbound.p, kb_.pt1.p, kb_.pseg.p, kb_.pw0.p, kb_.pw1.p, kb_.pw0_32.p,
-                                            kb_.pw1_32.p, kb_.pe.p, kb_.patom.p, kb_.pidx.p, rstart_b, rlen_b, nrow);
+                                            kb_.pw1_32.p, kb_.pe.p, kb_.patom.p, rstart_b, rlen_b, nrow);
     LSJK_CUDA(cudaGetLastError());
-    for (int a = 0; a < kNL; ++a)
-        for (int b = 0; b < kNL; ++b) {
-            long off = (long) (a * kNL + b) * nrow;
-            LSJK_CUDA(cudaMemcpyAsync(pl->kinv[a][b].row_start.p, rstart + off, sizeof(int) * nrow,
-                                      cudaMemcpyDeviceToDevice, s));
-            LSJK_CUDA(cudaMemcpyAsync(pl->kinv[a][b].row_len.p, rlen + off, sizeof(int) * nrow,
-                                      cudaMemcpyDeviceToDevice, s));
-        }
     LSJK_CUDA(cudaStreamSynchronize(s));
     pl->kinv_built = true;
     ctx->stats.kernel_launches += 20;
