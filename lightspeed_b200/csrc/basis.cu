@@ -205,6 +205,13 @@ void basis_init(Context* ctx, Basis* B)
     B->w0.assign(n, 1.0);
     B->w1.assign(n, 0.0);
     upload_prims(ctx, B);
+    std::vector<int> strip(B->ncart);
+    for (int P = 0; P < n; ++P) {
+        const int nc = ncart_count(B->L[P]);
+        // (the K kernels take shells up to f, so nc fits four bits wherever strip is read)
+        for (int k = 0; k < nc; ++k) strip[B->cart[P] + k] = B->cart[P] << 4 | (nc & 15);
+    }
+    B->dstrip.upload(strip, ctx->stream);
     {
         std::vector<int> t0(B->ncart), t1(B->ncart, -1);
         for (int k = 0; k < B->ncart; ++k) t0[k] = k;

@@ -148,6 +148,7 @@ struct Basis {
     DBuf<int> dL, dcart, dao;
     DBuf<int> dt0, dt1, dseg, datom;
     DBuf<double> dw0, dw1;
+    DBuf<int> dstrip;   // per Cartesian function: first function of its shell << 4 | functions of the shell
     // pure <-> cart maps: cart row -> (pure index, coef) and pure row -> (cart index, coef)
     DBuf<int> c2p_off, c2p_idx, p2c_off, p2c_idx;
     DBuf<double> c2p_w, p2c_w;

@@ -56,7 +56,11 @@ struct KArgs {
     BasisView b2, b4;         // indexed primitives (centres, cartIdx)
     const double* Dc[kMaxDens];  // D24 of each density of the build (Cartesian, ld4)
     int ld4;
-    double* Kc[kMaxDens];        // K13 of each density (Cartesian output space of bases 1 and 3, ld3)
+    // K13 of each density (Cartesian output space of bases 1 and 3, ld3): row-major in the FP64
+    // pass, in the FP32 pass in strip layout -- the N1 rows of a shell 1 from row c1 on are
+    // N1 x ld3 contiguous doubles, column by column, so element (c1 + a, col) stands at
+    // c1 * ld3 + col * N1 + a
+    double* Kc[kMaxDens];
     int ld3;
     int ng;                      // densities of the build, in groups of kKBatch (the tasks' grp)
     int nsub;                    // densities of a group / NG of the launch, rounded up: the launch

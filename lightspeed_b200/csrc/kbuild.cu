@@ -38,20 +38,37 @@ constexpr int kNCombo = kNL * kNL * kNL * kNL;
 
 
 
-// K = K + K^T in place (square ld x ld): the transposed half of the symmetric
-// D24 contributions, which the class kernels do not write.
-__global__ void k_symmetrize(double* __restrict__ K, int n)
+// The K of each density: row-major part and (mixed builds, else null) the FP32 pass's part in
+// strip layout.
+struct KParts {
+    double* row[kMaxDens];
+    const double* strip[kMaxDens];
+};
+
+// K = row + strip (KArgs::Kc; shell[r]: first row of r's shell << 4 | its rows), in place of
+// the row part, of density grid.y; with flip (square) also the transpose of that sum, the
+// half of the symmetric D24 contributions that the class kernels do not write.
+__global__ void k_finish(const __grid_constant__ KParts P, const int* __restrict__ shell, int n1, int n3, int flip)
 {
-    const long total = (long) n * n;
+    double* K = P.row[blockIdx.y];
+    const double* S = P.strip[blockIdx.y];
+    auto at = [&](int r, int c) {
+        double v = K[(long) r * n3 + c];
+        if (S) {
+            const int st = shell[r] >> 4, n = shell[r] & 15;
+            v += S[(long) st * n3 + (long) c * n + (r - st)];
+        }
+        return v;
+    };
+    const long total = (long) n1 * n3;
     for (long k = blockIdx.x * (long) blockDim.x + threadIdx.x; k < total; k += (long) gridDim.x * blockDim.x) {
-        const int i = (int) (k / n), j = (int) (k % n);
-        if (i > j) continue;
-        if (i == j) {
-            K[k] *= 2.0;
-        } else {
-            const double v = K[k] + K[(long) j * n + i];
+        const int r = (int) (k / n3), c = (int) (k % n3);
+        if (!flip) {
+            K[k] = at(r, c);
+        } else if (r <= c) {
+            const double v = at(r, c) + at(c, r);
             K[k] = v;
-            K[(long) j * n + i] = v;
+            K[(long) c * n3 + r] = v;
         }
     }
 }
@@ -277,7 +294,15 @@ void exchange_build(Context* ctx, const Ewald& ew, const PairList* pl12, const P
                     off[c + 1] = (cnt1[L1] && cnt3[L3]) ? (long) cnt2[L2] * cnt4[L4] * ngroup : 0L;
                 }
     for (int c = 0; c < kNCombo; ++c) off[c + 1] += off[c];
-    const bool mixed = ctx->precision == LSJK_PREC_MIXED && thredp > thresp;
+    // (the strips are indexed in 32 bits; a K of 2^32 elements runs in FP64 throughout)
+    const bool mixed = ctx->precision == LSJK_PREC_MIXED && thredp > thresp &&
+                       (unsigned long long) b1c * kb3->ncart < 0xffffffffull;
+    // K of the FP32 pass, in strip layout
+    double* strip[kMaxDens] = {};
+    for (int g = 0; mixed && g < ng; ++g) {
+        strip[g] = take<double>(ctx, (size_t) b1c * kb3->ncart);
+        LSJK_CUDA(cudaMemsetAsync(strip[g], 0, sizeof(double) * b1c * kb3->ncart, s));
+    }
     KTask* tasks = take<KTask>(ctx, off[kNCombo]);
     int* ntask = take<int>(ctx, 2 * kNCombo);   // all tasks, then the FP64-pass tasks
     KTask* tasks_hi = mixed ? take<KTask>(ctx, off[kNCombo]) : nullptr;
@@ -330,6 +355,7 @@ void exchange_build(Context* ctx, const Ewald& ew, const PairList* pl12, const P
     int lane = 0;
     // average partner-1 row of class L1: the entries' share of that shell's primitives
     const double rows12 = (double) pl12->kdat.nent / ((double) pl12->b1->nprim * b2->nprim);
+    const double stripe_len = pl12->npair < 2000 ? 2.0 : 8.0;
     // heaviest quartets first: their tails overlap the lighter classes
     for (int L1 = kNL - 1; L1 >= 0; --L1)
         for (int L2 = kNL - 1; L2 >= 0; --L2)
@@ -380,7 +406,7 @@ void exchange_build(Context* ctx, const Ewald& ew, const PairList* pl12, const P
                     A.flip = flip_ok ? 1 : 0;
                     A.gc = (pl12->b1->is_twin || pl34->b1->is_twin) ? 1 : 0;
                     A.sc = sc;
-                    A.split = (int) std::max(1.0, std::min(32.0, rows12 * cnt1[L1] / 2.0));
+                    A.split = (int) std::max(1.0, std::min(32.0, rows12 * cnt1[L1] / stripe_len));
                     A.nbin = kRysNbin[NR];
                     A.tmax = kRysTmax[NR];
                     A.status = ctx->status.p;
@@ -453,6 +479,7 @@ void exchange_build(Context* ctx, const Ewald& ew, const PairList* pl12, const P
                         A.thr_lo = thresp;
                         A.thr_hi = thredp;
                         A.split_hi = 0;
+                        for (int g = 0; g < ng; ++g) A.Kc[g] = strip[g];
                         A.rys = ctx->rys32.p + kRysOffset[NR];
                         A.asym_t = ctx->rys_asym32.p + NR * LSJK_RYS_NMAX;
                         A.asym_w = ctx->rys_asym32.p + (LSJK_RYS_NMAX + 1) * LSJK_RYS_NMAX + NR * LSJK_RYS_NMAX;
@@ -464,14 +491,17 @@ void exchange_build(Context* ctx, const Ewald& ew, const PairList* pl12, const P
                     }
                 }
     if (par) join_aux(ctx);
-    if (flip_ok) {
-        // basis 1 == basis 3 here, so each K13 is square
-        const int n = b3->ncart;
+    if (flip_ok || mixed) {
+        KParts P{};
         for (int g = 0; g < ng; ++g) {
-            k_symmetrize<<<std::min<long>(nblk((long) n * n, 256), 1184), 256, 0, s>>>(Kcart[g], n);
-            LSJK_CUDA(cudaGetLastError());
-            ctx->stats.kernel_launches++;
+            P.row[g] = Kcart[g];
+            P.strip[g] = strip[g];
         }
+        const long n = (long) b1c * b3->ncart;
+        k_finish<<<dim3((unsigned) std::min<long>(nblk(n, 256), 1184), ng), 256, 0, s>>>(P, kb1->dstrip.p, b1c, b3->ncart,
+                                                                                       flip_ok ? 1 : 0);
+        LSJK_CUDA(cudaGetLastError());
+        ctx->stats.kernel_launches++;
     }
 }
 

@@ -65,7 +65,7 @@ constexpr int kKGrab = 16;
 // partner-1 row serially for every 32 partners 3, so with one task per warp or less a
 // class takes as long as its longest rows ((p s|p s) of C10H22: 9% of the warps active
 // on average) and a small molecule's classes leave most of the GPU idle. The rows are
-// cut into up to KArgs::split stripes of two entries or more (a stripe repeats the
+// cut into up to KArgs::split stripes of eight entries or more (two in the smallest builds) (a stripe repeats the
 // task's header, D24 loads and segment flush).
 constexpr int kKUnitsPerWarp = 2;
 
@@ -82,6 +82,33 @@ struct alignas(16) KHdr {
     float wsym;             // 1/2 for a diagonal task of a symmetric D24, else 1
     int dbase, dn;          // densities dbase .. dbase + dn - 1 of the build (the task's sub-slot)
 };
+
+// Elements of a block that a flush stages at a time: all of a block up to nine, else the
+// largest divisor up to nine (a run of six doubles still covers most of two sectors).
+__host__ __device__ constexpr int k_flush_group(int nb)
+{
+    int g = nb < 9 ? nb : 9;
+    while (nb % g) --g;
+    return g;
+}
+
+// Staging of a segment flush of the FP32 pass, per warp: the active lanes' blocks one after
+// another, the position of each in K and (two-target partners 3) its weight. The FP32 pass
+// adds into K in strip layout (KArgs::Kc), where a block N1 x N3 is contiguous, consecutive
+// lanes adding consecutive elements: the L2 took 4.5e11 such reductions a second against
+// 1.9e11 with every lane adding to a sector of its own (a 2 MB target), and lanes without
+// a contribution cost no conversion and no reduction. (p s|p s) of C10H22 in FP32
+// 1.17 -> 0.58 ms. The FP64 pass flushes from the registers into the row-major K: staged, or
+// unstaged into strips (where a row's lanes share fewer sectors), C20H42 FP64 took 87.0
+// instead of 83.6 ms.
+template <typename R, int FG, bool W>
+struct KFlush {
+    R v[32 * FG];
+    unsigned base[32];
+    double wt[W ? 32 : 1];
+};
+template <typename R, bool W>
+struct KFlush<R, 0, W> {};   // straight from the registers
 
 // Lane l copies entry kb + l of the row (if it exists) into dst[l].
 template <typename R>
@@ -225,6 +252,10 @@ __global__ void __launch_bounds__(kKThreads) k_exchange(const __grid_constant__ 
     __shared__ __align__(8) uint64_t mbar;
     __shared__ KEnt<R> ring_all[kKWarps][2][32];
     __shared__ KHdr hdr_all[kKWarps][kKGrab];
+    constexpr int FG = k_flush_group(N1 * N3);
+    constexpr bool kStaged = !FP64 && N1 * N3 > 1;
+    __shared__ KFlush<R, kStaged ? FG : 0, G3 == 2> flush_all[kKWarps];
+    auto& fl = flush_all[threadIdx.x >> 5];
     const int ntask1 = *A.ntask;
     const int ntask_all = ntask1 * A.nsub;   // the task list once per density sub-slot
     // and once per partner-1 stripe
@@ -401,42 +432,66 @@ __global__ void __launch_bounds__(kKThreads) k_exchange(const __grid_constant__ 
                 int last_seg = k1a > 0 ? A.seg12[s12 + k1a - 1] : -1;
                 const float rmax = __int_as_float((int) __reduce_max_sync(
                     0xffffffffu, (unsigned) __float_as_int(in3 ? b34 / tlo : 0.0f)));   // (non-negative: ordered as bits)
-                // flush the finished shell segment of partner 1: one atomic per element, density
-                // and target pair (fire-and-forget reductions; a segmented shuffle sum over the
-                // lanes of one shell 3 before them measured slower)
+                // add the lanes' blocks v of shells c1, c3 (on: lanes that have one), times wt for a
+                // two-target partner 3
+                auto scatter = [&](double* Kc, const R* v, bool on, int c1, int c3t, double wt) {
+                    if constexpr (!kStaged) {
+                        if (on) {
+#pragma unroll
+                            for (int a = 0; a < N1; ++a) {
+                                double* row = Kc + (long) (c1 + a) * A.ld3 + c3t;
+#pragma unroll
+                                for (int c = 0; c < N3; ++c) {
+                                    const double x = wsym * (double) v[a * N3 + c];
+                                    atomicAdd(row + c, G3 == 2 ? wt * x : x);
+                                }
+                            }
+                        }
+                    } else {
+                        const unsigned m = __ballot_sync(0xffffffffu, on);
+                        const int nblk = __popc(m), at = __popc(m & ((1u << lane) - 1u));
+                        if (on) {
+                            fl.base[at] = (unsigned) c1 * A.ld3 + (unsigned) c3t * N1;
+                            if constexpr (G3 == 2) fl.wt[at] = wt;
+                        }
+#pragma unroll
+                        for (int e0 = 0; e0 < N1 * N3; e0 += FG) {
+                            if (on) {
+#pragma unroll
+                                for (int x = 0; x < FG; ++x)
+                                    fl.v[at * FG + x] = (R) wsym * v[((e0 + x) % N1) * N3 + (e0 + x) / N1];
+                            }
+                            __syncwarp();
+                            for (int e = lane; e < nblk * FG; e += 32) {
+                                const int k = e / FG;
+                                double x = (double) fl.v[e];
+                                if constexpr (G3 == 2) x *= fl.wt[k];
+                                atomicAdd(Kc + fl.base[k] + (e0 + e - k * FG), x);
+                            }
+                            __syncwarp();   // the next group (or flush) rewrites the staging
+                        }
+                    }
+                };
+                // flush the finished shell segment of partner 1 (all lanes; a segmented shuffle
+                // sum over the lanes of one shell 3 before it measured slower)
                 auto flush = [&]() {
-                    if (any) {
+                    if (kStaged ? __any_sync(0xffffffffu, any) : any) {
 #pragma unroll
                         for (int g = 0; g < NG; ++g) {
                             if (NG > 1 && g >= dn) break;   // (a pack of one density always has it)
                             double* Kc = A.Kc[dbase + g];
+                            auto targets = [&](int c1, R* v) {
+                                scatter(Kc, v, any, c1, c3, w30);
+                                if constexpr (G3 == 2) scatter(Kc, v, any && c3b >= 0, c1, c3b, w31);
 #pragma unroll
-                            for (int a = 0; a < N1; ++a)
+                                for (int t = 0; t < N1 * N3; ++t) v[t] = R(0);
+                            };
+                            targets(prev_c1, acc[g]);
+                            if constexpr (G1 == 2) {
+                                if (prev_c1b >= 0) targets(prev_c1b, accb[g]);
 #pragma unroll
-                                for (int c = 0; c < N3; ++c) {
-                                    const double v = wsym * (double) acc[g][a * N3 + c];
-                                    double* row = Kc + (long) (prev_c1 + a) * A.ld3;
-                                    if constexpr (G3 == 2) {
-                                        atomicAdd(row + c3 + c, w30 * v);
-                                        if (c3b >= 0) atomicAdd(row + c3b + c, w31 * v);
-                                    } else {
-                                        atomicAdd(row + c3 + c, v);
-                                    }
-                                    acc[g][a * N3 + c] = R(0);
-                                    if constexpr (G1 == 2) {
-                                        if (prev_c1b >= 0) {
-                                            const double vb = wsym * (double) accb[g][a * N3 + c];
-                                            double* rowb = Kc + (long) (prev_c1b + a) * A.ld3;
-                                            if constexpr (G3 == 2) {
-                                                atomicAdd(rowb + c3 + c, w30 * vb);
-                                                if (c3b >= 0) atomicAdd(rowb + c3b + c, w31 * vb);
-                                            } else {
-                                                atomicAdd(rowb + c3 + c, vb);
-                                            }
-                                        }
-                                        accb[g][a * N3 + c] = R(0);
-                                    }
-                                }
+                                for (int t = 0; t < N1 * N3; ++t) accb[g][t] = R(0);
+                            }
                         }
                     }
                     any = false;
