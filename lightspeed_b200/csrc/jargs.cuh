@@ -32,6 +32,8 @@ struct JArgs {
     long jbra_stride;         // distance between the densities' bra accumulators
     int nterm;
     double alpha[4], omega[4];
+    float alphaf[4], omegaf[4];     // the same in FP32
+    int bare;                       // bit tm: term tm is bare 1/r (omega = -1)
     float thresp;
 };
 

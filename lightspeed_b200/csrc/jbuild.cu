@@ -49,32 +49,39 @@ struct KetTables {
     int n[kNHerm], off[kNHerm];
 };
 
-// One launch for every class (grid.y). The key sorts by class, then by the screened
-// bound, largest first, dropped pairs last.
+// One launch for every class (grid.y), four lanes per pair (over the densities' block rows:
+// a batch of 36 densities took 380 us with a thread per pair). The key sorts by class, then
+// by the screened bound, largest first, dropped pairs last.
+constexpr int kScreenLanes = 4;
+
 __global__ void k_ket_screen(KetTables T, BasisView b3, BasisView b4, int symm, DSet D, float thre,
                              unsigned long long* __restrict__ key, int* __restrict__ val,
                              int* __restrict__ nkept, unsigned* __restrict__ maxbits)
 {
     const int cls = blockIdx.y;
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
+    const int thread = blockIdx.x * blockDim.x + threadIdx.x;
+    const int k = thread / kScreenLanes, sub = thread % kScreenLanes;
     bool keep = false;
     float B2 = 0.0f;
+    // max |D| over the pair block (both triangles if symmetric) and, for a
+    // batched launch, over its densities: the batch screens with the union
+    double v = 0.0;
     if (k < T.n[cls]) {
         int i = T.p1[cls][k], j = T.p2[cls][k];
         int a1 = b3.cart[i], a2 = b4.cart[j];
         int c1 = ncart_of(b3.L[i]), c2 = ncart_of(b4.L[j]);
         int ld = b4.ncart;
-        // max |D| over the pair block (both triangles if symmetric) and, for a
-        // batched launch, over its densities: the batch screens with the union
-        double v = 0.0;
-        for (int g = 0; g < D.n; ++g) {
+        for (int gx = sub; gx < D.n * c1; gx += kScreenLanes) {
+            const int g = gx / c1, x = gx - g * c1;
             const double* Dc = D.d[g];
-            for (int x = 0; x < c1; ++x)
-                for (int y = 0; y < c2; ++y) v = fmax(v, fabs(Dc[(long) (a1 + x) * ld + a2 + y]));
-            if (symm)
-                for (int x = 0; x < c1; ++x)
-                    for (int y = 0; y < c2; ++y) v = fmax(v, fabs(Dc[(long) (a2 + y) * ld + a1 + x]));
+            for (int y = 0; y < c2; ++y) {
+                v = fmax(v, fabs(Dc[(long) (a1 + x) * ld + a2 + y]));
+                if (symm) v = fmax(v, fabs(Dc[(long) (a2 + y) * ld + a1 + x]));
+            }
         }
+    }
+    for (int o = kScreenLanes / 2; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+    if (k < T.n[cls] && sub == 0) {
         B2 = (float) (v * (double) T.bound[cls][k]);
         keep = B2 > thre;
         key[T.off[cls] + k] = ((unsigned long long) cls << 32) | (keep ? ~__float_as_uint(B2) : 0xffffffffu);
@@ -195,7 +202,7 @@ __device__ void ket_record(int i, int j, BasisView b3, BasisView b4, bool symm, 
     rec[2] = Q[1];
     rec[3] = Q[2];
 #pragma unroll 1
-    for (int g = 0; g < DS.slots; ++g) {
+    for (int g = blockIdx.y; g < DS.slots; g += gridDim.y) {
         double* out = rec + 4 + g * H;
         if (g < DS.n)
             ket_herm_block<L3, L4>(E, DS.d[g], a1, a2, ld, symm, scale, pre, out);
@@ -204,6 +211,8 @@ __device__ void ket_record(int i, int j, BasisView b3, BasisView b4, bool symm, 
     }
 }
 
+// A thread per ket pair; the densities of a batch are shared out over grid.y (every slice
+// writes the same header).
 template <int LK>
 __global__ void k_ket_herm(const unsigned long long* __restrict__ keys_sorted, const int* __restrict__ perm,
                            const int* __restrict__ nkept, const int* __restrict__ p1, const int* __restrict__ p2,
@@ -226,9 +235,11 @@ __global__ void k_ket_herm(const unsigned long long* __restrict__ keys_sorted, c
     });
     (void) L4;
     if (rec32) {
+        constexpr int H = nherm_of(LK);
         float* r32 = rec32 + (long) k * S;
-#pragma unroll
-        for (int t = 0; t < S; ++t) r32[t] = (float) r[t];   // S is runtime: plain loop
+        for (int t = 0; t < 4; ++t) r32[t] = (float) r[t];
+        for (int g = blockIdx.y; g < Dc.slots; g += gridDim.y)
+            for (int t = 4 + g * H; t < 4 + (g + 1) * H; ++t) r32[t] = (float) r[t];
     }
 }
 
@@ -309,13 +320,22 @@ __device__ void bra_to_cart(int i, int j, BasisView b1, BasisView b2, bool symm,
         }
 }
 
+// The Cartesian J of each density of a build (grid.y) and the distance between the
+// densities' Hermite accumulators.
+struct JOut {
+    double* d[kMaxDens];
+    long stride;
+};
+
 template <int LB>
 __global__ void k_herm_to_cart(const int* __restrict__ nbra, const int* __restrict__ p1,
                                const int* __restrict__ p2, const double* __restrict__ geom,
                                BasisView b1, BasisView b2, int symm, const double* __restrict__ jbra,
-                               double* __restrict__ Jc)
+                               const __grid_constant__ JOut out)
 {
     constexpr int H = nherm_of(LB);
+    double* Jc = out.d[blockIdx.y];
+    jbra += blockIdx.y * out.stride;
     int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= *nbra) return;
     int i = p1[k], j = p2[k];
@@ -338,9 +358,11 @@ template <int LB>
 __global__ void k_herm_to_cart_warp(const int* __restrict__ nbra, const int* __restrict__ p1,
                                     const int* __restrict__ p2, const double* __restrict__ geom,
                                     BasisView b1, BasisView b2, int symm, const double* __restrict__ jbra,
-                                    double* __restrict__ Jc)
+                                    const __grid_constant__ JOut out)
 {
     constexpr int H = nherm_of(LB), V = LB + 1;
+    double* Jc = out.d[blockIdx.y];
+    jbra += blockIdx.y * out.stride;
     const int lane = threadIdx.x & 31;
     const long k = ((long) blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (k >= *nbra) return;   // whole warps leave together
@@ -681,7 +703,7 @@ KetSet prepare_kets(Context* ctx, const PairList* pl12, const PairList* pl34, co
     int* val = take<int>(ctx, total);
     int* perm = take<int>(ctx, total);
     if (total) {
-        k_ket_screen<<<dim3(nblk(nmax, 256), kNHerm), 256, 0, s>>>(KT, b3->view(), b4->view(), pl34->symm ? 1 : 0, DS,
+        k_ket_screen<<<dim3(nblk((long) nmax * kScreenLanes, 256), kNHerm), 256, 0, s>>>(KT, b3->view(), b4->view(), pl34->symm ? 1 : 0, DS,
                                                                   thre_ket, key, val, K.nket, maxbits);
         LSJK_CUDA(cudaGetLastError());
         // in double buffers: the sort then takes no second copy of its own from the scratch
@@ -706,7 +728,11 @@ KetSet prepare_kets(Context* ctx, const PairList* pl12, const PairList* pl34, co
         K.kbound[LK] = take<float>(ctx, n);
         const int off = KT.off[LK];
         auto herm = [&](auto lk) {
-            k_ket_herm<decltype(lk)::value><<<nblk(n, 128), 128, 0, s>>>(
+            // slices of the densities until there are two CTAs per multiprocessor (the 36
+            // (d|d) pairs of 8 H2O: 988 us for 36 densities in one slice)
+            const unsigned tiles = nblk(n, 128);
+            const unsigned ny = std::min<unsigned>(DS.slots, (2u * ctx->nsm + tiles - 1) / tiles);
+            k_ket_herm<decltype(lk)::value><<<dim3(tiles, ny), 128, 0, s>>>(
                 keys + off, perm + off, K.nket + LK, jk.p1.p, jk.p2.p, jk.geom.p, b3->view(), b4->view(), pl34->symm,
                 DS, krec, krec32, K.kbound[LK]);
         };
@@ -812,6 +838,9 @@ void coulomb_build(Context* ctx, const Ewald& ew, const PairList* pl12, const Pa
             for (int t = 0; t < A.nterm; ++t) {
                 A.alpha[t] = ew.alpha[t];
                 A.omega[t] = ew.omega[t];
+                A.alphaf[t] = (float) ew.alpha[t];
+                A.omegaf[t] = (float) ew.omega[t];
+                if (ew.omega[t] == -1.0) A.bare |= 1 << t;
             }
             A.thresp = thresp;
             auto launch = [&](const JArgs& X) {
@@ -861,27 +890,27 @@ void coulomb_build(Context* ctx, const Ewald& ew, const PairList* pl12, const Pa
     }
     if (par) join_aux(ctx);
 
-    // 5. back to Cartesian, per density
-    for (int g = 0; g < ng; ++g)
-        for (int LB = 0; LB < kNHerm; ++LB) {
-            const JBraClass& jb = pl12->jb[LB];
-            if (!jb.n) continue;
-            unsigned gr = nblk(jb.n, 128);
-            const double* jt = jbra[LB] + (long) g * jb.n * nherm_of(LB);
-            double* Jc = Jcart[g];
-            switch (LB) {
-            case 0: k_herm_to_cart<0><<<gr, 128, 0, s>>>(nbra + LB, jb.p1.p, jb.p2.p, jb.geom.p, b1->view(), b2->view(), pl12->symm, jt, Jc); break;
-            case 1: k_herm_to_cart<1><<<gr, 128, 0, s>>>(nbra + LB, jb.p1.p, jb.p2.p, jb.geom.p, b1->view(), b2->view(), pl12->symm, jt, Jc); break;
-            case 2: k_herm_to_cart<2><<<gr, 128, 0, s>>>(nbra + LB, jb.p1.p, jb.p2.p, jb.geom.p, b1->view(), b2->view(), pl12->symm, jt, Jc); break;
-            case 3: k_herm_to_cart_warp<3><<<nblk(jb.n, 4), 128, 0, s>>>(nbra + LB, jb.p1.p, jb.p2.p, jb.geom.p, b1->view(), b2->view(), pl12->symm, jt, Jc); break;
-            case 4: k_herm_to_cart_warp<4><<<nblk(jb.n, 4), 128, 0, s>>>(nbra + LB, jb.p1.p, jb.p2.p, jb.geom.p, b1->view(), b2->view(), pl12->symm, jt, Jc); break;
-            case 5: k_herm_to_cart_warp<5><<<nblk(jb.n, 4), 128, 0, s>>>(nbra + LB, jb.p1.p, jb.p2.p, jb.geom.p, b1->view(), b2->view(), pl12->symm, jt, Jc); break;
-            case 6: k_herm_to_cart_warp<6><<<nblk(jb.n, 4), 128, 0, s>>>(nbra + LB, jb.p1.p, jb.p2.p, jb.geom.p, b1->view(), b2->view(), pl12->symm, jt, Jc); break;
-            default: throw Error(LSJK_ENOTSUPP, "J: bra Hermite class above 6");
-            }
-            LSJK_CUDA(cudaGetLastError());
-            ctx->stats.kernel_launches++;
+    // 5. back to Cartesian, a launch per bra class for all densities
+    for (int LB = 0; LB < kNHerm; ++LB) {
+        const JBraClass& jb = pl12->jb[LB];
+        if (!jb.n) continue;
+        JOut out{};
+        for (int g = 0; g < ng; ++g) out.d[g] = Jcart[g];
+        out.stride = (long) jb.n * nherm_of(LB);
+        const dim3 thread(nblk(jb.n, 128), ng), warp(nblk(jb.n, 4), ng);
+        switch (LB) {
+        case 0: k_herm_to_cart<0><<<thread, 128, 0, s>>>(nbra + LB, jb.p1.p, jb.p2.p, jb.geom.p, b1->view(), b2->view(), pl12->symm, jbra[LB], out); break;
+        case 1: k_herm_to_cart<1><<<thread, 128, 0, s>>>(nbra + LB, jb.p1.p, jb.p2.p, jb.geom.p, b1->view(), b2->view(), pl12->symm, jbra[LB], out); break;
+        case 2: k_herm_to_cart<2><<<thread, 128, 0, s>>>(nbra + LB, jb.p1.p, jb.p2.p, jb.geom.p, b1->view(), b2->view(), pl12->symm, jbra[LB], out); break;
+        case 3: k_herm_to_cart_warp<3><<<warp, 128, 0, s>>>(nbra + LB, jb.p1.p, jb.p2.p, jb.geom.p, b1->view(), b2->view(), pl12->symm, jbra[LB], out); break;
+        case 4: k_herm_to_cart_warp<4><<<warp, 128, 0, s>>>(nbra + LB, jb.p1.p, jb.p2.p, jb.geom.p, b1->view(), b2->view(), pl12->symm, jbra[LB], out); break;
+        case 5: k_herm_to_cart_warp<5><<<warp, 128, 0, s>>>(nbra + LB, jb.p1.p, jb.p2.p, jb.geom.p, b1->view(), b2->view(), pl12->symm, jbra[LB], out); break;
+        case 6: k_herm_to_cart_warp<6><<<warp, 128, 0, s>>>(nbra + LB, jb.p1.p, jb.p2.p, jb.geom.p, b1->view(), b2->view(), pl12->symm, jbra[LB], out); break;
+        default: throw Error(LSJK_ENOTSUPP, "J: bra Hermite class above 6");
         }
+        LSJK_CUDA(cudaGetLastError());
+        ctx->stats.kernel_launches++;
+    }
 }
 
 // One bra-derivative pass of the J gradient: kets from Dket, bra pairs
@@ -939,6 +968,9 @@ static void coulomb_grad_bra(Context* ctx, const Ewald& ew, const PairList* pl, 
             for (int t = 0; t < A.nterm; ++t) {
                 A.alpha[t] = ew.alpha[t];
                 A.omega[t] = ew.omega[t];
+                A.alphaf[t] = (float) ew.alpha[t];
+                A.omegaf[t] = (float) ew.omega[t];
+                if (ew.omega[t] == -1.0) A.bare |= 1 << t;
             }
             A.thresp = thresp;
             OnAux on(ctx, lane++);

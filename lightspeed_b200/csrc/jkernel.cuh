@@ -26,10 +26,9 @@ __device__ __forceinline__ void j_quartet64(const JArgs& A, int g0, const double
     const double rs = rsqrt(p + q);
     const double rho = p * q * (rs * rs);
     for (int tm = 0; tm < A.nterm; ++tm) {
-        const double om = A.omega[tm];
         double d2 = 1.0, f = A.alpha[tm] * rs;
-        if (om != -1.0) {
-            const double w2 = om * om;
+        if (!(A.bare >> tm & 1)) {
+            const double om = A.omega[tm], w2 = om * om;
             d2 = w2 / (rho + w2);
             f *= sqrt(d2);
         }
@@ -67,11 +66,11 @@ constexpr float kBoysSwitch32 = (float) (LSJK_BOYS_TMAX - LSJK_BOYS_TMAX / LSJK_
 // evaluated in FP64 by its asymptotic form), added to the FP64 accumulators.
 template <int LB, int LK, int NG>
 __device__ __forceinline__ void j_quartet32(const JArgs& A, int g0, const float* tab, float p,
-                                            double Px, double Py, double Pz, double qd, double Qx, double Qy,
-                                            double Qz, const float* __restrict__ r32, double (*jp)[nherm_of(LB)])
+                                            double Px, double Py, double Pz, double Qx, double Qy, double Qz,
+                                            const float* __restrict__ r32, double (*jp)[nherm_of(LB)])
 {
     constexpr int L = LB + LK, HB = nherm_of(LB), HK = nherm_of(LK);
-    const float q = (float) qd;   // the FP32 record's q is this rounding
+    const float q = r32[0];
     const double Xd = Px - Qx, Yd = Py - Qy, Zd = Pz - Qz;
     const float X = (float) Xd, Y = (float) Yd, Z = (float) Zd;
     const float R2 = X * X + Y * Y + Z * Z;
@@ -83,10 +82,9 @@ __device__ __forceinline__ void j_quartet32(const JArgs& A, int g0, const float*
 #pragma unroll
         for (int t = 0; t < HB; ++t) jq[g][t] = 0.0f;
     for (int tm = 0; tm < A.nterm; ++tm) {
-        const float om = (float) A.omega[tm];
-        float d2 = 1.0f, f = (float) A.alpha[tm] * rs;
-        if (A.omega[tm] != -1.0) {
-            const float w2 = om * om;
+        float d2 = 1.0f, f = A.alphaf[tm] * rs;
+        if (!(A.bare >> tm & 1)) {
+            const float w2 = A.omegaf[tm] * A.omegaf[tm];
             d2 = w2 / (rho + w2);
             f *= sqrtf(d2);
         }
@@ -194,8 +192,7 @@ __global__ void __launch_bounds__(kJThreads) k_coulomb(JArgs A)
         } else if (__any_sync(0xffffffffu, pass)) {
             if (pass) {
                 nq32 += nd;
-                j_quartet32<LB, LK, NG>(A, g0, tab32, p32, Px, Py, Pz, qk, Qx, Qy, Qz, A.krec32 + (long) j * S,
-                                        jp);
+                j_quartet32<LB, LK, NG>(A, g0, tab32, p32, Px, Py, Pz, Qx, Qy, Qz, A.krec32 + (long) j * S, jp);
             }
         }
     }
