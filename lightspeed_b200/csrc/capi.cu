@@ -276,7 +276,16 @@ int lsjk_context_create(int device, lsjk_context** out)
             std::vector<double> asym(kRysAsymT, kRysAsymT + sizeof(kRysAsymT) / sizeof(double));
             asym.insert(asym.end(), kRysAsymW, kRysAsymW + sizeof(kRysAsymW) / sizeof(double));
             c.boys64.upload(boys, c.stream);
-            c.rys64.upload(rys, c.stream);
+            // FP64 rules: [root][bin][8] for t, then [root][bin][10] for w itself
+            std::vector<double> rys64;
+            const double* w64 = kRysW64;
+            for (int n = 1; n <= LSJK_RYS_NMAX; ++n) {
+                const long nt = (long) n * kRysNbin[n] * LSJK_TAB_NCOEF, nw = (long) n * kRysNbin[n] * LSJK_TAB_NCOEF_W64;
+                rys64.insert(rys64.end(), kRysCoef + kRysOffset[n], kRysCoef + kRysOffset[n] + nt);
+                rys64.insert(rys64.end(), w64, w64 + nw);
+                w64 += nw;
+            }
+            c.rys64.upload(rys64, c.stream);
             c.rys_asym64.upload(asym, c.stream);
             c.boys32.upload(std::vector<float>(boys.begin(), boys.end()), c.stream);
             c.rys32.upload(std::vector<float>(rys.begin(), rys.end()), c.stream);

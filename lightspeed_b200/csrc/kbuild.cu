@@ -431,7 +431,7 @@ void exchange_build(Context* ctx, const Ewald& ew, const PairList* pl12, const P
                     A.thr_lo = two_pass ? thredp : thresp;
                     A.thr_hi = inf;
                     A.split_hi = two_pass ? 1 : 0;
-                    A.rys = ctx->rys64.p + kRysOffset[NR];
+                    A.rys = ctx->rys64.p + kRysOffset64[NR];
                     A.asym_t = ctx->rys_asym64.p + NR * LSJK_RYS_NMAX;
                     A.asym_w = ctx->rys_asym64.p + (LSJK_RYS_NMAX + 1) * LSJK_RYS_NMAX + NR * LSJK_RYS_NMAX;
                     A.qcount = qcnt + c;
@@ -653,7 +653,7 @@ void exchange_grad_symm(Context* ctx, const Ewald& ew, const PairList* pl, const
                     }
                     const int NR = (L1 + L2 + L3 + L4 + 1) / 2 + 1;   // one quantum up
                     A.queue = queue + combo_index(L1, L2, L3, L4);
-                    A.rys = ctx->rys64.p + kRysOffset[NR];
+                    A.rys = ctx->rys64.p + kRysOffset64[NR];
                     A.asym_t = ctx->rys_asym64.p + NR * LSJK_RYS_NMAX;
                     A.asym_w = ctx->rys_asym64.p + (LSJK_RYS_NMAX + 1) * LSJK_RYS_NMAX + NR * LSJK_RYS_NMAX;
                     A.nbin = kRysNbin[NR];
@@ -767,7 +767,7 @@ void exchange_grad(Context* ctx, const Ewald& ew, const PairList* pl, const doub
                     A.G = G;
                     A.sc = sc;
                     A.thr_lo = thresp;
-                    A.rys = ctx->rys64.p + kRysOffset[NR];
+                    A.rys = ctx->rys64.p + kRysOffset64[NR];
                     A.asym_t = ctx->rys_asym64.p + NR * LSJK_RYS_NMAX;
                     A.asym_w = ctx->rys_asym64.p + (LSJK_RYS_NMAX + 1) * LSJK_RYS_NMAX + NR * LSJK_RYS_NMAX;
                     A.nbin = kRysNbin[NR];

@@ -264,7 +264,7 @@ __global__ void __launch_bounds__(kKThreads) k_exchange(const __grid_constant__ 
     // the grid is sized for the class's task capacity; CTAs whose warps cannot
     // get a task leave before staging the quadrature table
     if ((long) blockIdx.x * kKWarps >= ntask) return;
-    const unsigned bytes = (unsigned) (2 * NR * A.nbin * 8 * sizeof(R));
+    const unsigned bytes = (unsigned) (rys_block<R>(NR, A.nbin) * sizeof(R));
     if (!stage_bulk(tab, A.rys, bytes, &mbar, A.status)) return;
     const R* asym_t = static_cast<const R*>(A.asym_t);
     const R* asym_w = static_cast<const R*>(A.asym_w);
@@ -590,7 +590,7 @@ template <int L1, int L2, int L3, int L4, typename R, int NG, bool GC>
 void launch_k_one(Context* ctx, const KArgs& A, unsigned grid)
 {
     constexpr int NR = (L1 + L2 + L3 + L4) / 2 + 1;
-    const size_t smem = (size_t) 2 * NR * A.nbin * 8 * sizeof(R);
+    const size_t smem = (size_t) rys_block<R>(NR, A.nbin) * sizeof(R);
     // the shared-memory opt-in is a per-device function attribute: set it once per
     // device, and read how many CTAs of this kernel fit on a multiprocessor
     static std::atomic<unsigned long long> attr_devices{0};

@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(kXThreads) k_xgrad(const __grid_constant__ XGr
     double* tab = reinterpret_cast<double*>(xg_smem);
     __shared__ __align__(8) uint64_t mbar;
     __shared__ int queue_all[kXWarps][64];
-    if (!stage_bulk(tab, A.rys, (unsigned) (2 * NR * A.nbin * 8 * sizeof(double)), &mbar, A.status)) return;
+    if (!stage_bulk(tab, A.rys, (unsigned) (rys_block<double>(NR, A.nbin) * sizeof(double)), &mbar, A.status)) return;
     const int lane = threadIdx.x & 31;
     int* pend = queue_all[threadIdx.x >> 5];
     const float thre = A.sc->thre12;
@@ -459,7 +459,7 @@ void launch_one(Context* ctx, const XGradArgs& A0)
     A.nunit = (unsigned) nunit;
     size_t smem;
     if constexpr (lane)
-        smem = (size_t) 2 * ((L1 + L2 + L3 + L4 + 1) / 2 + 1) * A.nbin * 8 * sizeof(double);
+        smem = (size_t) rys_block<double>((L1 + L2 + L3 + L4 + 1) / 2 + 1, A.nbin) * sizeof(double);
     else
         smem = xwarp_warps<L1, L2, L3, L4>() * sizeof(XWarpTab<L1, L2, L3, L4>);
     constexpr int warps = lane ? kXWarps : xwarp_warps<L1, L2, L3, L4>();

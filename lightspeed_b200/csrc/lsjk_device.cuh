@@ -112,6 +112,35 @@ __device__ __forceinline__ double horner8(const double* __restrict__ c, double x
     return f;
 }
 
+// The same for the ten coefficients of the FP64 weight tables.
+__device__ __forceinline__ double horner10(const double* __restrict__ c, double x)
+{
+    const double2 c89 = reinterpret_cast<const double2*>(c)[4];
+    const double2 c01 = reinterpret_cast<const double2*>(c)[0];
+    const double2 c23 = reinterpret_cast<const double2*>(c)[1];
+    const double2 c45 = reinterpret_cast<const double2*>(c)[2];
+    const double2 c67 = reinterpret_cast<const double2*>(c)[3];
+    double f = c89.y;
+    f = fma(f, x, c89.x);
+    f = fma(f, x, c67.y);
+    f = fma(f, x, c67.x);
+    f = fma(f, x, c45.y);
+    f = fma(f, x, c45.x);
+    f = fma(f, x, c23.y);
+    f = fma(f, x, c23.x);
+    f = fma(f, x, c01.y);
+    f = fma(f, x, c01.x);
+    return f;
+}
+
+// Elements of one rule's table block: roots t, then weights (FP32: ln w in 8 coefficients;
+// FP64: w in 10, which costs two more operations than ln w and saves its exponential).
+template <typename R>
+__host__ __device__ constexpr int rys_block(int n, int nbin)
+{
+    return n * nbin * (sizeof(R) == 8 ? LSJK_TAB_NCOEF + LSJK_TAB_NCOEF_W64 : 2 * LSJK_TAB_NCOEF);
+}
+
 // Ampere-style asynchronous global -> shared copies of 4 / 8 bytes (one
 // thread each), grouped with commit/wait.
 __device__ __forceinline__ void cp_async4(void* smem, const void* gmem)
@@ -180,8 +209,9 @@ __device__ __forceinline__ void boys_eval(R T, const R* __restrict__ tab, R* __r
 }
 
 // Rys roots (returned as t^2) and weights of the N-point rule at T. `tab` is the
-// per-rule block [2N][nbin][8] (roots t, then ln w; for N = 1 the weight
-// w = F_0(T) itself, so the one-root classes need no exponential); `bscale` is
+// per-rule block: [N][nbin][8] for the roots t, then in FP32 [N][nbin][8] for ln w (for
+// N = 1 the weight w = F_0(T) itself, so the one-root classes need no exponential),
+// in FP64 [N][nbin][10] for w (rys_block); `bscale` is
 // nbin / tmax, formed once per thread and not divided out for every quartet;
 // `asym_t/asym_w` hold the half-range Gauss-Hermite limit used for T >= tmax.
 template <int N, typename R>
@@ -198,8 +228,12 @@ __device__ __forceinline__ void rys_eval(R T, const R* __restrict__ tab, int nbi
         for (int i = 0; i < N; ++i) {
             const R t = horner8(tab + 8 * (i * nbin + b), x);
             t2[i] = t * t;
-            const R lw = horner8(tab + 8 * ((N + i) * nbin + b), x);
-            w[i] = N == 1 ? lw : dexp(lw);
+            if constexpr (sizeof(R) == 8) {
+                w[i] = horner10(tab + 8 * N * nbin + LSJK_TAB_NCOEF_W64 * (i * nbin + b), x);
+            } else {
+                const R lw = horner8(tab + 8 * ((N + i) * nbin + b), x);
+                w[i] = N == 1 ? lw : dexp(lw);
+            }
         }
     } else {
         const R r = drsqrt(T);
@@ -270,8 +304,7 @@ __device__ __forceinline__ void rys_root(double T, const double* __restrict__ ta
         b = b < nbin - 1 ? b : nbin - 1;
         const double x = 2.0 * (u - b) - 1.0;
         t = horner8(tab + 8 * (i * nbin + b), x);
-        const double lw = horner8(tab + 8 * ((N + i) * nbin + b), x);
-        w = N == 1 ? lw : exp(lw);
+        w = horner10(tab + 8 * N * nbin + LSJK_TAB_NCOEF_W64 * (i * nbin + b), x);
     } else {
         const double r = rsqrt(T);
         t = asym_t[i] * r;

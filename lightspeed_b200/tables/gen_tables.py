@@ -35,6 +35,7 @@ NMAX_RYS = 9            # roots 1..9 (total angular momentum up to 16)
 MMAX_BOYS = 16          # Boys orders 0..16
 DEG = 7                 # polynomial degree per bin (8 coefficients)
 NCOEF = DEG + 1
+NCOEF_W64 = 10     # coefficients of the FP64 weight tables
 
 # Discretised Rys measure: positive half of a 1024-point Gauss-Legendre rule.
 _gx, _gw = legendre.leggauss(1024)
@@ -91,17 +92,17 @@ def boys_exact(mmax, T):
     return out
 
 
-def _fit_bins(func, nfun, tmax, nbin):
-    """Degree-DEG Chebyshev interpolation per bin, returned as monomial
+def _fit_bins(func, nfun, tmax, nbin, ncoef=NCOEF):
+    """Chebyshev interpolation of degree ncoef - 1 per bin, returned as monomial
     coefficients c[fun][bin][k] of sum_k c_k x^k, x in [-1, 1]."""
     h = tmax / nbin
-    xs = np.cos(np.pi * (np.arange(NCOEF) + 0.5) / NCOEF)  # Chebyshev nodes
-    coefs = np.zeros((nfun, nbin, NCOEF))
+    xs = np.cos(np.pi * (np.arange(ncoef) + 0.5) / ncoef)  # Chebyshev nodes
+    coefs = np.zeros((nfun, nbin, ncoef))
     for b in range(nbin):
         T0 = b * h
-        vals = np.array([func(T0 + 0.5 * h * (x + 1.0)) for x in xs])  # (NCOEF, nfun)
+        vals = np.array([func(T0 + 0.5 * h * (x + 1.0)) for x in xs])  # (ncoef, nfun)
         for f in range(nfun):
-            ch = chebyshev.chebfit(xs, vals[:, f], DEG)
+            ch = chebyshev.chebfit(xs, vals[:, f], ncoef - 1)
             coefs[f, b, :] = chebyshev.cheb2poly(ch)
     return coefs
 
@@ -145,6 +146,9 @@ def build_rys(n, width):
         return np.concatenate([t, w if n == 1 else np.log(w)])
 
     coefs = _fit_bins(func, 2 * n, tmax, nbin)
+    # the weights themselves for the FP64 kernels: degree 9 reaches the accuracy of ln w at
+    # degree 7 (2e-15 to 1e-14 relative for n = 2 to 7) and needs no exponential
+    wcoefs = _fit_bins(lambda T: rys_exact(n, T)[1], n, tmax, nbin, NCOEF_W64)
     # accuracy check on random points
     rng = np.random.default_rng(n)
     errt = errw = 0.0
@@ -153,7 +157,8 @@ def build_rys(n, width):
         v = _eval_bins(coefs, tmax, nbin, T)
         errt = max(errt, np.max(np.abs(v[:n] - t)))
         errw = max(errw, np.max(np.abs((v[n:] if n == 1 else np.exp(v[n:])) - w)))
-    return dict(n=n, tmax=tmax, nbin=nbin, coefs=coefs, asym=rys_asym(n), errt=errt, errw=errw)
+    return dict(n=n, tmax=tmax, nbin=nbin, coefs=coefs, wcoefs=wcoefs, asym=rys_asym(n), errt=errt,
+                errw=errw)
 
 
 def build_boys(width=0.25, tmax=36.0):
@@ -198,6 +203,14 @@ def write_inc(path, rys_list, boys):
     lines.append("static const long   kRysOffset[%d] = {0, %s};" % (NMAX_RYS + 2, ", ".join(str(o) for o in off)))
     allc = np.concatenate([np.concatenate([r["coefs"][:r["n"]].ravel(), r["coefs"][r["n"]:].ravel()]) for r in rys_list])
     lines.append("static const double kRysCoef[%d] = {\n%s};" % (len(allc), _fmt(allc)))
+    lines.append("// FP64 weights: per nrys, [root][bin][coef] for w, %d coefficients" % NCOEF_W64)
+    lines.append("#define LSJK_TAB_NCOEF_W64 %d" % NCOEF_W64)
+    wc = np.concatenate([r["wcoefs"].ravel() for r in rys_list])
+    lines.append("static const double kRysW64[%d] = {\n%s};" % (len(wc), _fmt(wc)))
+    off64 = [0]
+    for r in rys_list:
+        off64.append(off64[-1] + r["n"] * r["nbin"] * (NCOEF + NCOEF_W64))
+    lines.append("static const long   kRysOffset64[%d] = {0, %s};" % (NMAX_RYS + 2, ", ".join(str(o) for o in off64)))
     asym_t = np.zeros((NMAX_RYS + 1, NMAX_RYS))
     asym_w = np.zeros((NMAX_RYS + 1, NMAX_RYS))
     for r in rys_list:
