@@ -276,12 +276,13 @@ int lsjk_context_create(int device, lsjk_context** out)
             std::vector<double> asym(kRysAsymT, kRysAsymT + sizeof(kRysAsymT) / sizeof(double));
             asym.insert(asym.end(), kRysAsymW, kRysAsymW + sizeof(kRysAsymW) / sizeof(double));
             c.boys64.upload(boys, c.stream);
-            // FP64 rules: [root][bin][8] for t, then [root][bin][10] for w itself
+            // FP64 rules: [root][bin][8] for t, then [root][bin][10] for w itself (one root: [bin][8])
             std::vector<double> rys64;
             const double* w64 = kRysW64;
             for (int n = 1; n <= LSJK_RYS_NMAX; ++n) {
                 const long nt = (long) n * kRysNbin[n] * LSJK_TAB_NCOEF, nw = (long) n * kRysNbin[n] * LSJK_TAB_NCOEF_W64;
-                rys64.insert(rys64.end(), kRysCoef + kRysOffset[n], kRysCoef + kRysOffset[n] + nt);
+                rys64.insert(rys64.end(), kRysCoef + kRysOffset[n], kRysCoef + kRysOffset[n] + (n == 1 ? 2 * nt : nt));
+                if (n == 1) continue;
                 rys64.insert(rys64.end(), w64, w64 + nw);
                 w64 += nw;
             }

@@ -134,11 +134,12 @@ __device__ __forceinline__ double horner10(const double* __restrict__ c, double 
 }
 
 // Elements of one rule's table block: roots t, then weights (FP32: ln w in 8 coefficients;
-// FP64: w in 10, which costs two more operations than ln w and saves its exponential).
+// FP64: w in 10, which costs two more operations than ln w and saves its exponential; the
+// one-root rule has w in 8 in both: (ss|ss) of C20H42 6.7 ms, 8.0 ms with 10).
 template <typename R>
 __host__ __device__ constexpr int rys_block(int n, int nbin)
 {
-    return n * nbin * (sizeof(R) == 8 ? LSJK_TAB_NCOEF + LSJK_TAB_NCOEF_W64 : 2 * LSJK_TAB_NCOEF);
+    return n * nbin * (sizeof(R) == 8 && n > 1 ? LSJK_TAB_NCOEF + LSJK_TAB_NCOEF_W64 : 2 * LSJK_TAB_NCOEF);
 }
 
 // Ampere-style asynchronous global -> shared copies of 4 / 8 bytes (one
@@ -211,7 +212,7 @@ __device__ __forceinline__ void boys_eval(R T, const R* __restrict__ tab, R* __r
 // Rys roots (returned as t^2) and weights of the N-point rule at T. `tab` is the
 // per-rule block: [N][nbin][8] for the roots t, then in FP32 [N][nbin][8] for ln w (for
 // N = 1 the weight w = F_0(T) itself, so the one-root classes need no exponential),
-// in FP64 [N][nbin][10] for w (rys_block); `bscale` is
+// in FP64 [N][nbin][10] for w, N > 1 (rys_block); `bscale` is
 // nbin / tmax, formed once per thread and not divided out for every quartet;
 // `asym_t/asym_w` hold the half-range Gauss-Hermite limit used for T >= tmax.
 template <int N, typename R>
@@ -228,7 +229,7 @@ __device__ __forceinline__ void rys_eval(R T, const R* __restrict__ tab, int nbi
         for (int i = 0; i < N; ++i) {
             const R t = horner8(tab + 8 * (i * nbin + b), x);
             t2[i] = t * t;
-            if constexpr (sizeof(R) == 8) {
+            if constexpr (sizeof(R) == 8 && N > 1) {
                 w[i] = horner10(tab + 8 * N * nbin + LSJK_TAB_NCOEF_W64 * (i * nbin + b), x);
             } else {
                 const R lw = horner8(tab + 8 * ((N + i) * nbin + b), x);
@@ -292,7 +293,7 @@ __device__ __forceinline__ void rys_asym_pairs(float rho, float d2, float RR, fl
     }
 }
 
-// Root i alone of the N-point rule (FP64), for lanes that share a quartet's roots out.
+// Root i alone of the N-point rule (FP64, N > 1), for lanes that share a quartet's roots out.
 __device__ __forceinline__ void rys_root(double T, const double* __restrict__ tab, int N, int i, int nbin, double tmax,
                                          double bscale, const double* __restrict__ asym_t, const double* __restrict__ asym_w,
                                          double& t2, double& w)

@@ -147,7 +147,8 @@ def build_rys(n, width):
 
     coefs = _fit_bins(func, 2 * n, tmax, nbin)
     # the weights themselves for the FP64 kernels: degree 9 reaches the accuracy of ln w at
-    # degree 7 (2e-15 to 1e-14 relative for n = 2 to 7) and needs no exponential
+    # degree 7 (2e-15 to 1e-14 relative for n = 2 to 7) and needs no exponential (the one-point
+    # rule has its w at degree 7 above)
     wcoefs = _fit_bins(lambda T: rys_exact(n, T)[1], n, tmax, nbin, NCOEF_W64)
     # accuracy check on random points
     rng = np.random.default_rng(n)
@@ -203,13 +204,13 @@ def write_inc(path, rys_list, boys):
     lines.append("static const long   kRysOffset[%d] = {0, %s};" % (NMAX_RYS + 2, ", ".join(str(o) for o in off)))
     allc = np.concatenate([np.concatenate([r["coefs"][:r["n"]].ravel(), r["coefs"][r["n"]:].ravel()]) for r in rys_list])
     lines.append("static const double kRysCoef[%d] = {\n%s};" % (len(allc), _fmt(allc)))
-    lines.append("// FP64 weights: per nrys, [root][bin][coef] for w, %d coefficients" % NCOEF_W64)
+    lines.append("// FP64 weights: per nrys > 1, [root][bin][coef] for w, %d coefficients" % NCOEF_W64)
     lines.append("#define LSJK_TAB_NCOEF_W64 %d" % NCOEF_W64)
-    wc = np.concatenate([r["wcoefs"].ravel() for r in rys_list])
+    wc = np.concatenate([r["wcoefs"].ravel() for r in rys_list if r["n"] > 1])
     lines.append("static const double kRysW64[%d] = {\n%s};" % (len(wc), _fmt(wc)))
     off64 = [0]
     for r in rys_list:
-        off64.append(off64[-1] + r["n"] * r["nbin"] * (NCOEF + NCOEF_W64))
+        off64.append(off64[-1] + r["n"] * r["nbin"] * (NCOEF + (NCOEF_W64 if r["n"] > 1 else NCOEF)))
     lines.append("static const long   kRysOffset64[%d] = {0, %s};" % (NMAX_RYS + 2, ", ".join(str(o) for o in off64)))
     asym_t = np.zeros((NMAX_RYS + 1, NMAX_RYS))
     asym_w = np.zeros((NMAX_RYS + 1, NMAX_RYS))
