@@ -430,8 +430,11 @@ __global__ void __launch_bounds__(kKThreads) k_exchange(const __grid_constant__ 
                 // a stripe may start inside a shell segment, whose largest bound came before it:
                 // its first entry is then not taken for the segment's
                 int last_seg = k1a > 0 ? A.seg12[s12 + k1a - 1] : -1;
-                const float rmax = __int_as_float((int) __reduce_max_sync(
-                    0xffffffffu, (unsigned) __float_as_int(in3 ? b34 / tlo : 0.0f)));   // (non-negative: ordered as bits)
+                // (the ratios are non-negative, so they are ordered as their bits; tlo = 0, a threshold of
+                // zero or below, passes everything: infinite, not the NaN of 0 / 0 where b34 underflowed)
+                const float ratio = in3 ? (tlo > 0.0f ? b34 / tlo : __int_as_float(0x7f800000)) : 0.0f;
+                const float rmax =
+                    __int_as_float((int) __reduce_max_sync(0xffffffffu, (unsigned) __float_as_int(ratio)));
                 // add the lanes' blocks v of shells c1, c3 (on: lanes that have one), times wt for a
                 // two-target partner 3
                 auto scatter = [&](double* Kc, const R* v, bool on, int c1, int c3t, double wt) {
@@ -511,7 +514,8 @@ __global__ void __launch_bounds__(kKThreads) k_exchange(const __grid_constant__ 
                     const int kend = min(32, n12 - kb);
                     // the chunk's entries, one per lane: those that may pass for some lane (b12 times
                     // the warp's largest b34 / tlo, with room for the roundings; each lane still applies
-                    // its exact screen), and those that start a shell segment
+                    // its exact screen; a zero b12 against an infinite ratio may pass, hence the
+                    // negated test), and those that start a shell segment
                     float bl = 0.0f;
                     int sl = -1;
                     if (lane < kend) {
@@ -521,7 +525,7 @@ __global__ void __launch_bounds__(kKThreads) k_exchange(const __grid_constant__ 
                     int sp = __shfl_up_sync(0xffffffffu, sl, 1);
                     if (lane == 0) sp = last_seg;
                     last_seg = __shfl_sync(0xffffffffu, sl, kend - 1);
-                    const bool cand = bl >= thre12 && bl * rmax >= 0.999999f;
+                    const bool cand = bl >= thre12 && !(bl * rmax < 0.999999f);
                     unsigned todo = __ballot_sync(0xffffffffu, lane < kend && cand);
                     // segments are ordered by their largest (first) bound: where one's first entry
                     // cannot pass, nothing later does
