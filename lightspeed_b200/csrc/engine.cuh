@@ -261,7 +261,7 @@ struct Context {
     // over them (fork after the shared set-up, join before the back
     // transforms), so one class's tail overlaps the next class's start
     static constexpr int kAux = 16;
-    int naux = kAux;                // the ones in use between fork_aux and join_aux
+    int naux = kAux;                // the ones in use while an AuxFork lives
     cudaStream_t aux[kAux] = {};
     cudaEvent_t fork_ev = nullptr;
     cudaEvent_t join_ev[kAux] = {};
@@ -305,25 +305,44 @@ inline char* Context::scratch_take(size_t bytes)
     return scratch.back()->p;
 }
 
-// Make the auxiliary streams wait for the work enqueued so far on ctx->stream. Each stream
-// costs three host calls per build (about 5 us), which a small molecule's build feels: with
-// 16 instead of 8, one H2O/6-31G* J+K build took 913 instead of 613 us, while the class
-// kernels of C10H22/cc-pVDZ overlapped better (27.0 -> 25.1 ms).
-inline void fork_aux(Context* ctx, long npair)
-{
-    ctx->naux = npair < 20000 ? 8 : Context::kAux;
-    LSJK_CUDA(cudaEventRecord(ctx->fork_ev, ctx->stream));
-    for (int i = 0; i < ctx->naux; ++i) LSJK_CUDA(cudaStreamWaitEvent(ctx->aux[i], ctx->fork_ev, 0));
-}
-
-// Make ctx->stream wait for everything enqueued on the auxiliary streams.
-inline void join_aux(Context* ctx)
-{
-    for (int i = 0; i < ctx->naux; ++i) {
-        LSJK_CUDA(cudaEventRecord(ctx->join_ev[i], ctx->aux[i]));
-        LSJK_CUDA(cudaStreamWaitEvent(ctx->stream, ctx->join_ev[i], 0));
+// The auxiliary streams of one build, from the fork (they wait for the work enqueued so far
+// on ctx->stream) to the join (ctx->stream waits for everything enqueued on them). A build
+// that throws in between joins on the way out: what it had launched still reads the scratch
+// that the context's next call takes over. Each stream costs three host calls per build
+// (about 5 us), which a small molecule's build feels: with 16 instead of 8, one H2O/6-31G*
+// J+K build took 913 instead of 613 us, while the class kernels of C10H22/cc-pVDZ overlapped
+// better (27.0 -> 25.1 ms).
+class AuxFork {
+public:
+    AuxFork(Context* c, long npair) : ctx(c), main(c->stream)
+    {
+        ctx->naux = npair < 20000 ? 8 : Context::kAux;
+        LSJK_CUDA(cudaEventRecord(ctx->fork_ev, main));
+        for (int i = 0; i < ctx->naux; ++i) LSJK_CUDA(cudaStreamWaitEvent(ctx->aux[i], ctx->fork_ev, 0));
     }
-}
+    AuxFork(const AuxFork&) = delete;
+    AuxFork& operator=(const AuxFork&) = delete;
+    void join()
+    {
+        for (int i = 0; i < ctx->naux; ++i) {
+            LSJK_CUDA(cudaEventRecord(ctx->join_ev[i], ctx->aux[i]));
+            LSJK_CUDA(cudaStreamWaitEvent(main, ctx->join_ev[i], 0));
+        }
+        joined = true;
+    }
+    ~AuxFork()
+    {
+        if (joined) return;
+        for (int i = 0; i < ctx->naux; ++i)   // (an error here changes nothing: one is on its way already)
+            if (cudaEventRecord(ctx->join_ev[i], ctx->aux[i]) == cudaSuccess)
+                (void) cudaStreamWaitEvent(main, ctx->join_ev[i], 0);
+    }
+
+private:
+    Context* ctx;
+    cudaStream_t main;
+    bool joined = false;
+};
 
 // While alive, ctx->stream is auxiliary stream i (the launchers enqueue on
 // ctx->stream); restores the main stream on exit.

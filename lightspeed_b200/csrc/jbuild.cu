@@ -795,7 +795,8 @@ void coulomb_build(Context* ctx, const Ewald& ew, const PairList* pl12, const Pa
     // class kernels go round-robin to the auxiliary streams (not while the
     // autotuner times them one by one)
     const bool par = !ctx->tuning;
-    if (par) fork_aux(ctx, std::max(pl12->npair, pl34->npair));
+    std::optional<AuxFork> fork;
+    if (par) fork.emplace(ctx, std::max(pl12->npair, pl34->npair));
     int lane = 0;
     for (int LB = 0; LB < kNHerm; ++LB) {
         const JBraClass& jb = pl12->jb[LB];
@@ -888,7 +889,7 @@ void coulomb_build(Context* ctx, const Ewald& ew, const PairList* pl12, const Pa
             launch(A);
         }
     }
-    if (par) join_aux(ctx);
+    if (fork) fork->join();
 
     // 5. back to Cartesian, a launch per bra class for all densities
     for (int LB = 0; LB < kNHerm; ++LB) {
@@ -932,7 +933,7 @@ static void coulomb_grad_bra(Context* ctx, const Ewald& ew, const PairList* pl, 
         LSJK_CUDA(cudaMemsetAsync(vbras[LB], 0, sizeof(double) * nv, s));
     }
     // class kernels go round-robin to the auxiliary streams, as in the J build
-    fork_aux(ctx, pl->npair);
+    AuxFork kernels(ctx, pl->npair);
     int lane = 0;
     for (int LB = 0; LB < kNHerm; ++LB) {
         const JBraClass& jb = pl->jb[LB];
@@ -986,8 +987,8 @@ static void coulomb_grad_bra(Context* ctx, const Ewald& ew, const PairList* pl, 
             }
         }
     }
-    join_aux(ctx);
-    fork_aux(ctx, pl->npair);
+    kernels.join();
+    AuxFork back(ctx, pl->npair);
     for (int LB = 0; LB < kNHerm; ++LB) {
         const JBraClass& jb = pl->jb[LB];
         if (!jb.n) continue;
@@ -1008,7 +1009,7 @@ static void coulomb_grad_bra(Context* ctx, const Ewald& ew, const PairList* pl, 
         LSJK_CUDA(cudaGetLastError());
         ctx->stats.kernel_launches++;
     }
-    join_aux(ctx);
+    back.join();
 }
 
 // E = sum D12 (12|34) D34 moves with all four centres: its gradient is the

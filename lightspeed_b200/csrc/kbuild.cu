@@ -351,7 +351,8 @@ void exchange_build(Context* ctx, const Ewald& ew, const PairList* pl12, const P
     // class kernels go round-robin to the auxiliary streams (not while the
     // autotuner times them one by one)
     const bool par = !ctx->tuning;
-    if (par) fork_aux(ctx, std::max(pl12->npair, pl34->npair));
+    std::optional<AuxFork> fork;
+    if (par) fork.emplace(ctx, std::max(pl12->npair, pl34->npair));
     int lane = 0;
     // average partner-1 row of class L1: the entries' share of that shell's primitives
     const double rows12 = (double) pl12->kdat.nent / ((double) pl12->b1->nprim * b2->nprim);
@@ -490,7 +491,7 @@ void exchange_build(Context* ctx, const Ewald& ew, const PairList* pl12, const P
                         launch_k1(ctx, A, cap, L1, L2, L3, L4, true);
                     }
                 }
-    if (par) join_aux(ctx);
+    if (fork) fork->join();
     if (flip_ok || mixed) {
         KParts P{};
         for (int g = 0; g < ng; ++g) {
@@ -637,7 +638,7 @@ void exchange_grad_symm(Context* ctx, const Ewald& ew, const PairList* pl, const
         off[L1][L2][side] = (int) pl->cls_off[c];
         cnt[L1][L2][side] = (int) (pl->cls_off[c + 1] - pl->cls_off[c]);
     }
-    fork_aux(ctx, pl->npair);
+    AuxFork fork(ctx, pl->npair);
     int lane = 0;
     // heaviest classes first, so their tails overlap the lighter ones
     for (int L1 = kNL - 1; L1 >= 0; --L1)
@@ -661,7 +662,7 @@ void exchange_grad_symm(Context* ctx, const Ewald& ew, const PairList* pl, const
                     OnAux on(ctx, lane++);
                     launch_xgrad(ctx, A, L1, L2, L3, L4);
                 }
-    join_aux(ctx);
+    fork.join();
     k_xsum<<<nblk(ng, 128), 128, 0, s>>>(copies, kCopies, ng, G);
     LSJK_CUDA(cudaGetLastError());
     ctx->stats.kernel_launches++;

@@ -216,7 +216,8 @@ void one_electron(Context* ctx, int kind, const PairList* pl, const Ewald* ew, c
     if (ew && ew->alpha.size() > 4) throw Error(LSJK_EINVAL, "IntBox::potential: at most 4 Ewald terms");
     // the classes of V overlap on the auxiliary streams; those of S and T are too short to
     const bool par = kind == kOneV;
-    if (par) fork_aux(ctx, pl->npair);
+    std::optional<AuxFork> fork;
+    if (par) fork.emplace(ctx, pl->npair);
     for (size_t c = 0; c + 1 < pl->cls_off.size(); ++c) {
         OneArgs A{};
         A.p1 = pl->p1.p;
@@ -248,7 +249,7 @@ void one_electron(Context* ctx, int kind, const PairList* pl, const Ewald* ew, c
             launch_one<kOneS>(ctx, A, LA, LB);
         }
     }
-    if (par) join_aux(ctx);
+    if (fork) fork->join();
 }
 
 } // namespace lsjk
