@@ -86,25 +86,6 @@ __device__ __forceinline__ XBra load_bra(const XGradArgs& A, int i)
     return b;
 }
 
-// Work unit -> bra index and ket range. Units run chunk by chunk over all bras,
-// the ket chunks with the largest bounds (the most quartets) first.
-struct XUnit {
-    int i, j0, j1;
-};
-
-__device__ __forceinline__ XUnit unit_of(const XGradArgs& A, unsigned unit)
-{
-    XUnit u;
-    const int nb = A.bn[0] + A.bn[1];
-    const int c = (int) (unit / (unsigned) nb), bi = (int) (unit % (unsigned) nb);
-    u.i = bi < A.bn[0] ? A.boff[0] + bi : A.boff[1] + bi - A.bn[0];
-    const int nc0 = (A.kn[0] + A.chunk - 1) / A.chunk;
-    const int s = c < nc0 ? 0 : 1, cs = c - (s ? nc0 : 0);
-    u.j0 = A.koff[s] + cs * A.chunk;
-    u.j1 = A.koff[s] + min(A.kn[s], (cs + 1) * A.chunk);
-    return u;
-}
-
 // Adds the bra's sums to this CTA's copy of G.
 __device__ __forceinline__ void add_bra(const XGradArgs& A, const XBra& b, int lane, const double gA[3],
                                         const double gB[3])
@@ -448,22 +429,19 @@ void launch_one(Context* ctx, const XGradArgs& A0)
     constexpr bool lane = XG<L1, L2, L3, L4>::lane;
     const long nb = (long) A.bn[0] + A.bn[1], nk = (long) A.kn[0] + A.kn[1];
     if (nb == 0 || nk == 0) return;
-    // kets per work unit: a few units per warp of the GPU where there are that many pairs of
-    // pairs, within [32, 2048] (a partial last batch of a unit wastes lanes) for a quartet per
-    // lane and [4, 256] for a quartet per warp
-    const long units = 16L * ctx->nsm * kXWarps;
-    const long lo = lane ? 32 : 4, hi = lane ? 2048 : 256;
-    A.chunk = (int) std::min(hi, std::max(lo, (nb * nk / units + lo - 1) / lo * lo));
-    const long nunit = nb * ((A.kn[0] + A.chunk - 1) / A.chunk + (A.kn[1] + A.chunk - 1) / A.chunk);
-    if (nunit > 0x7fffffffL) throw Error(LSJK_EINVAL, "K gradient: too many pairs");
-    A.nunit = (unsigned) nunit;
+    // a few units per warp of the GPU, [32, 2048] kets each (a partial last batch of a unit
+    // wastes lanes) for a quartet per lane and [4, 256] for a quartet per warp
+    const XSplit split =
+        xgrad_split(nb, A.kn[0], A.kn[1], lane ? 32 : 4, lane ? 2048 : 256, 16L * ctx->nsm * kXWarps);
+    A.chunk = split.chunk;
+    A.nunit = split.nunit;
     size_t smem;
     if constexpr (lane)
         smem = (size_t) rys_block<double>((L1 + L2 + L3 + L4 + 1) / 2 + 1, A.nbin) * sizeof(double);
     else
         smem = xwarp_warps<L1, L2, L3, L4>() * sizeof(XWarpTab<L1, L2, L3, L4>);
     constexpr int warps = lane ? kXWarps : xwarp_warps<L1, L2, L3, L4>();
-    const unsigned grid = (unsigned) std::min<long>((nunit + warps - 1) / warps, 8L * ctx->nsm);
+    const unsigned grid = (unsigned) std::min<long>(((long) A.nunit + warps - 1) / warps, 8L * ctx->nsm);
     auto run = [&](auto kern) {
         // the shared-memory opt-in is a per-device function attribute: set it once per device
         static std::atomic<unsigned long long> devices{0};
