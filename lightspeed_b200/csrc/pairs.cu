@@ -111,15 +111,15 @@ __global__ void k_gather_pairs(const PairTmp* __restrict__ in, const int* __rest
 __global__ void k_class_starts(const unsigned long long* __restrict__ key, int n, int ncls, int* __restrict__ start,
                                unsigned* __restrict__ low)
 {
-    const int c = threadIdx.x;
-    if (c > ncls) return;
-    int lo = 0, hi = n;
-    while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if ((key[mid] >> 32) < (unsigned long long) c) lo = mid + 1; else hi = mid;
+    for (int c = threadIdx.x; c <= ncls; c += blockDim.x) {
+        int lo = 0, hi = n;
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if ((key[mid] >> 32) < (unsigned long long) c) lo = mid + 1; else hi = mid;
+        }
+        start[c] = c == ncls ? n : lo;
+        low[c] = lo < n ? (unsigned) key[lo] : 0u;
     }
-    start[c] = c == ncls ? n : lo;
-    low[c] = lo < n ? (unsigned) key[lo] : 0u;
 }
 
 // Gaussian product geometry of a pair: p = e1 + e2, P = (e1 A + e2 B) / p.
@@ -332,44 +332,45 @@ void build_pairlist(Context* ctx, PairList* pl)
     unsigned long long* k2s = take<unsigned long long>(ctx, n);
     int* perm = take<int>(ctx, n);
     k_keys_cls_bound<<<nblk(n, 256), 256, 0, s>>>(tmp, perm1, n, 0, k2);
-    radix_sort_pairs(ctx, k2, k2s, perm1, perm, n, 40);
+    // (any angular momentum: J and K refuse shells above f themselves)
+    const int ncls = (b1->maxL + 1) * nL2, nherm = b1->maxL + b2->maxL + 1;
+    int class_bits = 8;
+    while (std::max(ncls, nherm) > 1 << class_bits) ++class_bits;
+    radix_sort_pairs(ctx, k2, k2s, perm1, perm, n, 32 + class_bits);
     k_gather_pairs<<<nblk(n, 256), 256, 0, s>>>(tmp, perm, n, pl->p1.p, pl->p2.p, pl->bound.p);
     LSJK_CUDA(cudaGetLastError());
 
     // class offsets and the leading (largest) bound of each class
-    constexpr int kMaxCls = 128;   // (s to n shells on either side)
-    const int ncls = (b1->maxL + 1) * nL2, nherm = b1->maxL + b2->maxL + 1;
-    if (ncls >= kMaxCls || nherm >= kMaxCls)
-        throw Error(LSJK_ENOTSUPP, "PairList: angular momentum above d is not supported by the GPU J/K kernels");
-    int* starts = take<int>(ctx, 4 * kMaxCls);
-    unsigned* lows = reinterpret_cast<unsigned*>(starts + 2 * kMaxCls);
-    k_class_starts<<<1, kMaxCls, 0, s>>>(k2s, (int) n, ncls, starts, lows);
+    const int ns = ncls + nherm + 2;   // starts of the classes, then of the Hermite classes
+    int* starts = take<int>(ctx, 2 * ns);
+    unsigned* lows = reinterpret_cast<unsigned*>(starts + ns);
+    k_class_starts<<<1, 128, 0, s>>>(k2s, (int) n, ncls, starts, lows);
 
     // J bra view: stable re-sort of pass-1 order by (L1+L2, bound desc)
     int* perm_h = take<int>(ctx, n);
     k_keys_herm<<<nblk(n, 256), 256, 0, s>>>(tmp, perm1, n, b1->dL.p, b2->dL.p, k2);
-    radix_sort_pairs(ctx, k2, k2s, perm1, perm_h, n, 40);
-    k_class_starts<<<1, kMaxCls, 0, s>>>(k2s, (int) n, nherm, starts + kMaxCls, lows + kMaxCls);
+    radix_sort_pairs(ctx, k2, k2s, perm1, perm_h, n, 32 + class_bits);
+    k_class_starts<<<1, 128, 0, s>>>(k2s, (int) n, nherm, starts + ncls + 1, lows + ncls + 1);
     k_gather_pairs<<<nblk(n, 256), 256, 0, s>>>(tmp, perm_h, n, pl->jall.p1.p, pl->jall.p2.p, pl->jall.bound.p);
     k_pair_geom<<<nblk(n, 256), 256, 0, s>>>(b1->view(), b2->view(), pl->jall.p1.p, pl->jall.p2.p, (int) n,
                                             pl->jall.geom.p);
     LSJK_CUDA(cudaGetLastError());
-    int hst[4 * kMaxCls];
-    LSJK_CUDA(cudaMemcpyAsync(hst, starts, sizeof(hst), cudaMemcpyDeviceToHost, s));
+    std::vector<int> hst(2 * ns);
+    LSJK_CUDA(cudaMemcpyAsync(hst.data(), starts, sizeof(int) * hst.size(), cudaMemcpyDeviceToHost, s));
     LSJK_CUDA(cudaStreamSynchronize(s));
     for (int c = 0; c < ncls; ++c) {
         if (hst[c + 1] == hst[c]) continue;
         if (hst[c] > 0) pl->cls_off.push_back(hst[c]);
         pl->cls_L1.push_back(c / nL2);
         pl->cls_L2.push_back(c % nL2);
-        const unsigned bits = ~(unsigned) hst[2 * kMaxCls + c];
+        const unsigned bits = ~(unsigned) hst[ns + c];
         float b;
         memcpy(&b, &bits, sizeof(b));
         pl->cls_max.push_back(b);
         pl->max_bound = std::max(pl->max_bound, (double) b);
     }
     pl->cls_off.push_back(n);
-    const int* hh = hst + kMaxCls;
+    const int* hh = hst.data() + ncls + 1;
     for (int h = 0; h < nherm; ++h) {
         const int st = hh[h], cnt = hh[h + 1] - st;
         if (h >= kNHerm) {
