@@ -11,7 +11,7 @@ import pytest
 
 from oracle import ref
 
-pytestmark = pytest.mark.gpu
+pytestmark = [pytest.mark.gpu, pytest.mark.skipif(not ref.available(), reason="oracle/_ref/libls_ref.so not built")]
 
 
 def test_one_electron_vs_oracle(ls, golden_dir):
