@@ -76,14 +76,17 @@ struct DBuf {
     ~DBuf() { release(); }
     void alloc(size_t count) {
         release();
-        n = count;
         if (count == 0) return;
         g_device_allocations.fetch_add(1, std::memory_order_relaxed);
         cudaError_t e = cudaMalloc(&p, sizeof(T) * count);
         if (e != cudaSuccess) {
+            // left empty, so that no later call takes a piece of a block that is not there, and
+            // the runtime's last error cleared, so that the next launch check does not find it
             p = nullptr;
+            (void) cudaGetLastError();
             throw Error(LSJK_ENOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
         }
+        n = count;
     }
     void upload(const std::vector<T>& h, cudaStream_t s) {
         alloc(h.size());
@@ -299,8 +302,9 @@ inline char* Context::scratch_take(size_t bytes)
     }
     if (scratch_fixed) throw Error(LSJK_ENOMEM, "fixed scratch block exhausted");
     size_t sz = std::max(bytes, size_t(64) << 20);
-    scratch.emplace_back(new DBuf<char>());
-    scratch.back()->alloc(sz);
+    std::unique_ptr<DBuf<char>> blk(new DBuf<char>());
+    blk->alloc(sz);   // (may throw: the scratch then stays as it was)
+    scratch.push_back(std::move(blk));
     scratch_used = used + bytes;
     return scratch.back()->p;
 }
