@@ -273,6 +273,7 @@ struct Context {
     size_t scratch_used = 0;
     bool scratch_fixed = false;     // scratch is a caller-independent fixed block: never grow
     char* scratch_take(size_t bytes);
+    bool scratch_take_all(size_t bytes, int count, char** out);
     void scratch_reset() { scratch_used = 0; }
     int smem_optin = 0;
     int nsm = 148;                  // multiprocessors of the device
@@ -307,6 +308,21 @@ inline char* Context::scratch_take(size_t bytes)
     scratch.push_back(std::move(blk));
     scratch_used = used + bytes;
     return scratch.back()->p;
+}
+
+// `count` pieces of `bytes`, or none where they do not all fit (false, the scratch as it was).
+inline bool Context::scratch_take_all(size_t bytes, int count, char** out)
+{
+    const size_t used = scratch_used, blocks = scratch.size();
+    try {
+        for (int k = 0; k < count; ++k) out[k] = scratch_take(bytes);
+    } catch (const Error& e) {
+        if (e.code != LSJK_ENOMEM) throw;
+        scratch.resize(blocks);
+        scratch_used = used;
+        return false;
+    }
+    return true;
 }
 
 // The auxiliary streams of one build, from the fork (they wait for the work enqueued so far

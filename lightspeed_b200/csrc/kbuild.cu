@@ -295,18 +295,21 @@ void exchange_build(Context* ctx, const Ewald& ew, const PairList* pl12, const P
                 }
     for (int c = 0; c < kNCombo; ++c) off[c + 1] += off[c];
     // (the strips are indexed in 32 bits; a K of 2^32 elements runs in FP64 throughout)
-    const bool mixed = ctx->precision == LSJK_PREC_MIXED && thredp > thresp &&
-                       (unsigned long long) b1c * kb3->ncart < 0xffffffffull;
-    // K of the FP32 pass, in strip layout
-    double* strip[kMaxDens] = {};
-    for (int g = 0; mixed && g < ng; ++g) {
-        strip[g] = take<double>(ctx, (size_t) b1c * kb3->ncart);
-        LSJK_CUDA(cudaMemsetAsync(strip[g], 0, sizeof(double) * b1c * kb3->ncart, s));
-    }
+    bool mixed = ctx->precision == LSJK_PREC_MIXED && thredp > thresp &&
+                 (unsigned long long) b1c * kb3->ncart < 0xffffffffull;
     KTask* tasks = take<KTask>(ctx, off[kNCombo]);
     int* ntask = take<int>(ctx, 2 * kNCombo);   // all tasks, then the FP64-pass tasks
     KTask* tasks_hi = mixed ? take<KTask>(ctx, off[kNCombo]) : nullptr;
     unsigned* queue = take<unsigned>(ctx, 2 * kNCombo);   // per class and pass (one launch each)
+    // K of the FP32 pass, in strip layout: the last thing taken, so that where the device has no
+    // room for it the build runs in FP64 throughout in the memory that this takes
+    char* strip[kMaxDens] = {};
+    const size_t strip_bytes = sizeof(double) * b1c * kb3->ncart;
+    if (mixed && !ctx->scratch_take_all(strip_bytes, ng, strip)) {
+        mixed = false;
+        std::fill(strip, strip + kMaxDens, nullptr);
+    }
+    for (int g = 0; mixed && g < ng; ++g) LSJK_CUDA(cudaMemsetAsync(strip[g], 0, strip_bytes, s));
     unsigned long long* qcnt = ctx->counters.p + kNJClass;                          // FP64 K classes
     unsigned long long* qcnt32 = ctx->counters.p + kNJClass + kNKClass + kNJClass;  // FP32 K classes
     LSJK_CUDA(cudaMemsetAsync(ntask, 0, sizeof(int) * 2 * kNCombo, s));
@@ -480,7 +483,7 @@ void exchange_build(Context* ctx, const Ewald& ew, const PairList* pl12, const P
                         A.thr_lo = thresp;
                         A.thr_hi = thredp;
                         A.split_hi = 0;
-                        for (int g = 0; g < ng; ++g) A.Kc[g] = strip[g];
+                        for (int g = 0; g < ng; ++g) A.Kc[g] = reinterpret_cast<double*>(strip[g]);
                         A.rys = ctx->rys32.p + kRysOffset[NR];
                         A.asym_t = ctx->rys_asym32.p + NR * LSJK_RYS_NMAX;
                         A.asym_w = ctx->rys_asym32.p + (LSJK_RYS_NMAX + 1) * LSJK_RYS_NMAX + NR * LSJK_RYS_NMAX;
@@ -496,7 +499,7 @@ void exchange_build(Context* ctx, const Ewald& ew, const PairList* pl12, const P
         KParts P{};
         for (int g = 0; g < ng; ++g) {
             P.row[g] = Kcart[g];
-            P.strip[g] = strip[g];
+            P.strip[g] = reinterpret_cast<const double*>(strip[g]);
         }
         const long n = (long) b1c * b3->ncart;
         k_finish<<<dim3((unsigned) std::min<long>(nblk(n, 256), 1184), ng), 256, 0, s>>>(P, kb1->dstrip.p, b1c, b3->ncart,

@@ -10,7 +10,6 @@ from host_code import compile_host, source_part
 FAKE = """
 #include <atomic>
 #include <cstdint>
-#include <cstdlib>
 #include <functional>
 #include <memory>
 #include <stdexcept>
@@ -25,7 +24,9 @@ std::vector<std::pair<char*, size_t>> live;
 template <typename T> int cudaMalloc(T** p, size_t n)
 {
     if (given + (long) n > room) return last_error = 2;   // (*p is left as it was)
-    *p = (T*) std::malloc(1);
+    static uintptr_t next = 1 << 20;   // addresses only: nothing reads or writes there
+    *p = (T*) next;
+    next += n;
     live.push_back({(char*) *p, n});
     given += n;
     return 0;
@@ -33,7 +34,7 @@ template <typename T> int cudaMalloc(T** p, size_t n)
 int cudaFree(void* p)
 {
     for (size_t k = 0; k < live.size(); ++k)
-        if (live[k].first == p) { given -= live[k].second; live.erase(live.begin() + k); std::free(p); return 0; }
+        if (live[k].first == p) { given -= live[k].second; live.erase(live.begin() + k); return 0; }
     return last_error = 1;
 }
 int cudaGetLastError() { const int e = last_error; last_error = 0; return e; }
@@ -53,6 +54,7 @@ struct Context {
     size_t scratch_used = 0;
     bool scratch_fixed = false;
     char* scratch_take(size_t bytes);
+    bool scratch_take_all(size_t bytes, int count, char** out);
     void scratch_reset() { scratch_used = 0; }
 };
 """
@@ -74,6 +76,23 @@ extern "C" int take(long bytes)
     } catch (const Error& e) {
         return e.code != LSJK_ENOMEM ? -3 : (cudaGetLastError() ? -4 : 0);
     }
+}
+// 1: all of them, apart from one another; 0: none, and the scratch as it was
+extern "C" int take_all(long bytes, int count)
+{
+    std::vector<char*> p(count);
+    const size_t used = c->scratch_used;
+    const long before = given;
+    if (!c->scratch_take_all(bytes, count, p.data()))
+        return used == c->scratch_used && given == before && !cudaGetLastError() ? 0 : -1;
+    for (int k = 0; k < count; ++k) {
+        bool there = false;
+        for (auto& q : live) there = there || (p[k] >= q.first && p[k] + bytes <= q.first + q.second);
+        if (!there) return -2;
+        for (int j = 0; j < k; ++j)
+            if (p[k] < p[j] + bytes && p[j] < p[k] + bytes) return -3;
+    }
+    return 1;
 }
 """
 
@@ -108,3 +127,15 @@ def test_calls_after_a_refused_one(lib):
     lib.reset()
     assert [lib.take(L(60 * MB)) for _ in range(3)] == [1, 1, 1]
     assert lib.held() <= 300 * MB
+
+
+def test_all_or_none(lib):
+    L = ctypes.c_long
+    lib.start(L(300 * MB))
+    assert lib.take(L(70 * MB)) == 1
+    assert lib.take_all(L(50 * MB), 3) == 1
+    assert lib.take_all(L(30 * MB), 3) == 0
+    assert lib.take(L(14 * MB)) == 1           # the rest of a block is still there
+    lib.reset()
+    assert lib.take_all(L(50 * MB), 4) == 1
+    assert lib.take_all(L(100 * MB), 3) == 0
