@@ -1,10 +1,11 @@
 // Internal data structures of the B200 J/K engine (not part of the C ABI).
 //
-// Device memory layout (all arrays in HBM, one allocation each):
+// Device memory layout (all arrays in HBM):
 //  * Basis: per-primitive SoA (c, e, x, y, z, L, cartIdx, ...), plus the
 //    pure<->Cartesian maps of its shells as CSR rows.
 //  * PairList: the Schwarz-screened primitive pairs sorted exactly like the
-//    reference PairList (class (L1,L2), bound desc, prim1 asc, prim2 asc).
+//    reference PairList (class (L1,L2), bound desc, prim1 asc, prim2 asc);
+//    its arrays are slices of one allocation, the K-invert rows' of another.
 //    Two derived views are kept next to it:
 //      - JBra: pairs merged by Hermite angular momentum L1+L2 and re-sorted by
 //        bound, with the Gaussian-product geometry (p, P) precomputed;
@@ -56,7 +57,7 @@ struct Error : std::runtime_error {
 // cudaMalloc goes through DBuf::alloc); read by lsjk_device_allocations().
 inline std::atomic<long> g_device_allocations{0};
 
-// Device buffer owned by RAII (freed with the context's stream-ordered pool).
+// Device buffer owned by RAII, or a slice of one that outlives it.
 template <typename T>
 struct DBuf {
     T* p = nullptr;
@@ -329,9 +330,17 @@ inline bool Context::scratch_take_all(size_t bytes, int count, char** out)
 // on ctx->stream) to the join (ctx->stream waits for everything enqueued on them). A build
 // that throws in between joins on the way out: what it had launched still reads the scratch
 // that the context's next call takes over. Each stream costs three host calls per build
-// (about 5 us), which a small molecule's build feels: with 16 instead of 8, one H2O/6-31G*
-// J+K build took 913 instead of 613 us, while the class kernels of C10H22/cc-pVDZ overlapped
-// better (27.0 -> 25.1 ms).
+// (about 5 us), which the smallest builds feel, and the class kernels of larger ones overlap
+// better on more streams. J+K builds with 8 and with 16 streams, FP64 / mixed, us:
+//   1 H2O/6-31G* (261 pairs)        678 / 1076       711 / 1145
+//   2 H2O (752)                     669 / 953        587 / 874
+//   4 H2O (2256)                   1180 / 1581      1056 / 1421
+//   8 H2O (6670)                   3480 / 4025      3477 / 3896
+//   C6H14/cc-pVDZ (11836)          8902 / 9044      9060 / 8941
+//   C10H22 (22857)                21650 / 19661    21709 / 19504
+//   C20H42 (50417)                61837 / 52553    62079 / 52356
+// So the line at 20000 pairs is not the best one for mixed builds (from 8 H2O to C20H42 they gain
+// 0.4 to 3%) nor for two to four waters (10%); one water wants eight.
 class AuxFork {
 public:
     AuxFork(Context* c, long npair) : ctx(c), main(c->stream)

@@ -359,6 +359,12 @@ void exchange_build(Context* ctx, const Ewald& ew, const PairList* pl12, const P
     int lane = 0;
     // average partner-1 row of class L1: the entries' share of that shell's primitives
     const double rows12 = (double) pl12->kdat.nent / ((double) pl12->b1->nprim * b2->nprim);
+    // entries a stripe has at least, and 32 stripes per task at most. FP64 J+K builds with 2, 4,
+    // 8 and 16 entries, us: 1 H2O/6-31G* 673, 685, 663, 709; 2 H2O 669, 691, 709, 853; CH4/cc-pVDZ
+    // 697, 709, 720, 910; 4 H2O (2256 pairs) 1220, 1163, 1186, 1243; C3H8 2571, 2474, 2458, 2507;
+    // 8 H2O 3627, 3524, 3480, 3452; 16 H2O 11823, 11752, 11714, 11549; C20H42 within 0.5% of one
+    // another. Without stripes 732, 856, 918, 1434, 2919, 3728, 11545 and (C20H42) the same; 8 or
+    // 64 stripes at most instead of 32: within 3% everywhere.
     const double stripe_len = pl12->npair < 2000 ? 2.0 : 8.0;
     // heaviest quartets first: their tails overlap the lighter classes
     for (int L1 = kNL - 1; L1 >= 0; --L1)

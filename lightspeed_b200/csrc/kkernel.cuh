@@ -65,8 +65,8 @@ constexpr int kKGrab = 16;
 // partner-1 row serially for every 32 partners 3, so with one task per warp or less a
 // class takes as long as its longest rows ((p s|p s) of C10H22: 9% of the warps active
 // on average) and a small molecule's classes leave most of the GPU idle. The rows are
-// cut into up to KArgs::split stripes of eight entries or more (two in the smallest builds) (a stripe repeats the
-// task's header, D24 loads and segment flush).
+// cut into up to KArgs::split stripes (exchange_build says how short they may be; a stripe
+// repeats the task's header, D24 loads and segment flush).
 constexpr int kKUnitsPerWarp = 2;
 
 // Everything a task needs before its partner rows, prepared by one lane per

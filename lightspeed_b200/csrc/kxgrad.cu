@@ -24,10 +24,10 @@
 // of 32 runs as one batch, a quartet per lane, whatever the pass rate was.
 //
 // Bound by the FP64 pipe and its latency at 8 warps per multiprocessor (the
-// straight-line quartets use 128-255 registers). Measured, J and K gradient
-// through the host API: C10H22/cc-pVDZ with a density of converged extent
-// 391 -> 29.1 ms (K kernels 366 -> 20 ms), (H2O)2/cc-pVTZ 66.6 -> 21.8 ms
-// (K kernels 42 -> 10 ms), against one quartet per ordered (1,2,3,4) and warp.
+// straight-line quartets use 128-255 registers). Measured, the K gradient alone
+// through the host API, against the general routine on the same density (one
+// quartet per ordered (1,2,3,4) and warp): C10H22/cc-pVDZ with a density of
+// converged extent 20.1 against 371 ms, (H2O)2/cc-pVTZ 2.5 against 40.2 ms.
 #include <algorithm>
 #include <atomic>
 #include "engine.cuh"

@@ -271,7 +271,8 @@ static __constant__ RysAsymPairs c_rys_asym_pairs = make_rys_asym_pairs();
 // T = rho d2 RR, rounded to FP32 once: T, 1/T and 1/sqrt(T) are carried as unevaluated
 // sums of two floats (products split exactly by fma; one Newton step on the hardware
 // rsqrt, whose residual e = 1 - T r^2 ~ 2^-22 is itself exact to ~2^-47). The results
-// equal the FP64 evaluation rounded to FP32 to within 2^-24 (1 + 1e-5) relative. In FP64
+// equal the FP64 evaluation rounded to FP32 in all but 5 of 1.5e7 samples and are within
+// 2^-24 (1 + 1e-5) of 64 bits, as that is, for any rsqrt good to 2 ulp. In FP64
 // this took eight conversions and a dozen FP64 operations per quartet: half the
 // conversion pipe's load of the light classes.
 template <int N>
