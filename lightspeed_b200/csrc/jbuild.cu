@@ -820,18 +820,18 @@ void coulomb_build(Context* ctx, const Ewald& ew, const PairList* pl12, const Pa
             A.boys32 = ctx->boys32.p + (long) (LB + LK) * LSJK_BOYS_NBIN * 8;
             A.mixed = mixed ? 1 : 0;
             A.thredp = thredp;
-            if (ctx->tune.j_chunk[LB][LK] > 0) {
-                A.chunk = ctx->tune.j_chunk[LB][LK];
-                A.tuned = 1;
-            } else {
-                // default: kJChunk kets per CTA, halved (down to 8) while the grid would not
-                // give every multiprocessor two CTAs: a thread walks its chunk serially, so a
-                // small molecule's kernel takes as long as one chunk
-                const long tiles = (jb.n + kJThreads - 1) / kJThreads;
-                int chunk = kJChunk;
-                while (chunk > 8 && tiles * ((jk.n + chunk - 1) / chunk) < 2L * ctx->nsm) chunk >>= 1;
-                A.chunk = chunk;
-            }
+            // default: kJChunk kets per CTA, halved (down to 8) while the grid would not
+            // give every multiprocessor two CTAs: a thread walks its chunk serially, so a
+            // small molecule's kernel takes as long as one chunk
+            const long tiles = (jb.n + kJThreads - 1) / kJThreads;
+            int default_chunk = kJChunk;
+            while (default_chunk > 8 && tiles * ((jk.n + default_chunk - 1) / default_chunk) < 2L * ctx->nsm)
+                default_chunk >>= 1;
+            auto set_chunk = [&](JArgs& X, int c) {   // c: a table entry (0: the default)
+                X.chunk = c > 0 ? c : default_chunk;
+                X.tuned = c > 0;
+            };
+            set_chunk(A, ctx->tune.j_chunk[LB][LK]);
             A.ng = ng;
             A.slots = DS.slots;
             A.jbra_stride = (long) jb.n * nherm_of(LB);
@@ -857,15 +857,14 @@ void coulomb_build(Context* ctx, const Ewald& ew, const PairList* pl12, const Pa
                 }
             };
             if (ctx->tuning) {
-                // autotuner: time the candidate ket chunk sizes on scratch outputs
-                static const int cand[] = {128, 256, 512, 1024, 2048, 4096};
+                // autotuner: time the default and the candidate ket chunk sizes on scratch outputs
+                static const int cand[] = {0, 128, 256, 512, 1024, 2048, 4096};
                 JArgs T = A;
                 T.jbra = take<double>(ctx, (long) DS.slots * jb.n * nherm_of(LB));
                 T.qcount = T.qcount32 = ctx->tune_sink.p;
                 float best = 1e30f;
                 for (int c : cand) {
-                    T.chunk = c;
-                    T.tuned = 1;
+                    set_chunk(T, c);
                     float ms = 1e30f;
                     for (int rep = 0; rep < 2; ++rep) {
                         LSJK_CUDA(cudaEventRecord(ctx->ev0, s));
@@ -881,8 +880,7 @@ void coulomb_build(Context* ctx, const Ewald& ew, const PairList* pl12, const Pa
                         ctx->tune.j_chunk[LB][LK] = c;
                     }
                 }
-                A.chunk = ctx->tune.j_chunk[LB][LK];
-                A.tuned = 1;
+                set_chunk(A, ctx->tune.j_chunk[LB][LK]);
             }
             std::optional<OnAux> on;
             if (par) on.emplace(ctx, lane++);
